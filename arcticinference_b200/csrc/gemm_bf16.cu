@@ -42,13 +42,16 @@ constexpr int kBlockK = 64;  // bf16 elements: one 128-byte swizzle atom per row
 constexpr int kBlockKFp8 = 128;  // e4m3 elements in the same 128 bytes
 constexpr int kBlockKBytes = 128;
 constexpr int kUmmaK = 16;
-constexpr int kGemmThreads = 192;
+// Warps: TMA, MMA, then eight for the epilogue, two per TMEM lane quadrant that take alternate
+// 64-column groups.
+constexpr int kEpilogueWarps = 8;
+constexpr int kGemmThreads = (2 + kEpilogueWarps) * 32;
 constexpr int kMaxStages = 8;
 constexpr uint32_t kABytes = kBlockM * kBlockK * 2;
-// Per-epilogue-warp staging tile for coalesced stores: 32 rows x 64 bf16, rows padded to 144
-// bytes so that the 16-byte accesses of eight lanes fall in distinct banks both ways.
-constexpr int kStoreStagePitch = 144;
-constexpr int kStoreStageBytes = 32 * kStoreStagePitch;
+// Per-epilogue-warp staging tile for coalesced loads and stores: 32 rows x 64 bf16, the 16-byte
+// chunks of a row XORed with the row so that eight lanes hit distinct banks both ways.
+constexpr int kStoreStageBytes = 32 * 128;
+constexpr int kStoreBytes = kEpilogueWarps * kStoreStageBytes;
 
 struct GemmArgs {
   int rows_a, rows_b, K;
@@ -99,6 +102,21 @@ struct GemmArgs {
   TailSignal sig;
 };
 
+__device__ __forceinline__ uint32_t stage_chunk(int row, int chunk) {
+  return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4));
+}
+
+// Adds eight bf16 values to eight floats.
+__device__ __forceinline__ void add8(float (&v)[8], const uint4& q) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const float2 f = __bfloat1622float2(h[u]);
+    v[2 * u] += f.x;
+    v[2 * u + 1] += f.y;
+  }
+}
+
 __device__ __forceinline__ float gelu_erf(float x) {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
@@ -136,12 +154,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* store_stage = reinterpret_cast<uint8_t*>(bars) + 256;
-  // the tile's per-column scales, fetched while the k-loop runs (a lone tile per CTA pays for
-  // every load that waits until the accumulator is complete)
-  // (one private copy per epilogue warp, so that no barrier between warps is involved)
-  float* col_scale = reinterpret_cast<float*>(store_stage + 4 * kStoreStageBytes) +
-                     ((threadIdx.x >> 5) & 3) * 256;
-
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bars_base = smem_u32(bars);
   auto full_bar = [&](int s) { return bars_base + 8u * s; };
@@ -162,7 +174,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 4);
+      mbar_init(tempty_bar(a), kEpilogueWarps);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -301,80 +313,80 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
-      const uint32_t idesc =
-          p.fp8 ? make_idesc(kBlockM, (uint32_t)p.bn, 0, 0, 0, 0)
-                : make_idesc(kBlockM, (uint32_t)p.bn, 1, 1, 0, p.b_mn_major ? 1u : 0u);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
-        int tile_a, tile_b, split;
-        decode_work(p, w, tile_a, tile_b, split);
-        const int kb0 = split * p.kblocks_per_split;
-        const int kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, 200 + acc, w)) break;
+    // The whole warp walks the loop with warp-uniform values and one elected lane issues:
+    // descriptors then live in uniform registers and an instruction goes out as fast as the
+    // tensor core takes it (64 cycles at N = 128, 128 at N = 256; from a branch of one thread every
+    // 186 cycles whatever its shape).
+    const uint32_t idesc =
+        p.fp8 ? make_idesc(kBlockM, (uint32_t)p.bn, 0, 0, 0, 0)
+              : make_idesc(kBlockM, (uint32_t)p.bn, 1, 1, 0, p.b_mn_major ? 1u : 0u);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint64_t a0 = make_desc_kmajor_sw128(smem_base);
+    const uint64_t b0 = p.b_mn_major ? make_desc_mnmajor_sw128(smem_base + kABytes, 8192u)
+                                     : make_desc_kmajor_sw128(smem_base + kABytes);
+    const uint64_t stage_step = stage_bytes / 16;
+    // K-major: 16 bf16 or 32 e4m3 (32 bytes) further inside the swizzle atom = +2 in the
+    // encoded address; MN-major: 16 rows of 128 bytes further = +128.
+    const uint64_t b_step = p.b_mn_major ? 128u : 2u;
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+      int tile_a, tile_b, split;
+      decode_work(p, w, tile_a, tile_b, split);
+      const int kb0 = split * p.kblocks_per_split;
+      const int kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
+      if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                                             200 + acc, w)))
+        break;
+      tc_fence_after();
+      const uint32_t d_tmem = tm + (uint32_t)acc * acc_stride;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag, p.status,
+                                               300 + stage, kb))) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)acc * acc_stride;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag, p.status, 300 + stage, kb)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_base + (uint32_t)stage * stage_bytes;
-          const uint64_t a_desc = make_desc_kmajor_sw128(a_addr);
-          const uint64_t b_desc = p.b_mn_major ? make_desc_mnmajor_sw128(a_addr + kABytes, 8192u)
-                                               : make_desc_kmajor_sw128(a_addr + kABytes);
-          // K-major: 16 bf16 or 32 e4m3 (32 bytes) further inside the swizzle atom = +2 in the
-          // encoded address; MN-major: 16 rows of 128 bytes further = +128.
-          const uint64_t b_step = p.b_mn_major ? 128u : 2u;
+        const uint64_t a_desc = a0 + (uint64_t)stage * stage_step;
+        const uint64_t b_desc = b0 + (uint64_t)stage * stage_step;
+        if (elect_one()) {
           if (p.fp8) {
 #pragma unroll
-            for (int k = 0; k < kBlockKBytes / 32; ++k) {
+            for (int k = 0; k < kBlockKBytes / 32; ++k)
               umma_f8_ss(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc,
                          (kb > kb0 || k > 0) ? 1u : 0u);
-            }
           } else {
 #pragma unroll
-            for (int k = 0; k < kBlockK / kUmmaK; ++k) {
+            for (int k = 0; k < kBlockK / kUmmaK; ++k)
               umma_f16_ss(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + b_step * (uint64_t)k, idesc,
                           (kb > kb0 || k > 0) ? 1u : 0u);
-            }
           }
           tc_commit(empty_bar(stage));
-          if (++stage == p.stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (kb == kb1 - 1) tc_commit(tfull_bar(acc));
         }
-        if (!ok) break;
-        tc_commit(tfull_bar(acc));
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        __syncwarp();
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
     }
   } else {
     // --------------------------------- epilogue --------------------------------
     pdl_wait();  // scales, bias and residual come from earlier kernels; the output may still be read by one
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
+    const int half = (warp - 2) >> 2;  // which of the quadrant's two warps this is
     const int row = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool scaled = p.scale_a != nullptr && !p.out_f32;
     if (p.cluster_splits > 1) {
       // one work item per CTA; what follows the accumulator is the cluster exchange below
-      if (scaled) {
-        const int cw = p.bn / p.cluster_splits;
-        int ta, tb, sp;
-        decode_work(p, (int)blockIdx.x, ta, tb, sp);
-        const long long c0 = (long long)tb * p.bn + (long long)sp * cw;
-        for (int i = lane; i < cw; i += 32)
-          col_scale[i] = (c0 + i < p.rows_b) ? p.scale_b[c0 + i] : 0.f;
-        __syncwarp();
-      }
       cluster_acc_ok = mbar_wait(tfull_bar(0), 0, abort_flag, p.status, 400, (int)blockIdx.x);
       tc_fence_after();
     } else
@@ -385,12 +397,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const bool row_ok = a_row < p.rows_a;
       const long long b0 = (long long)tile_b * p.bn;
       const float sa = (scaled && row_ok) ? p.scale_a[a_row] : 1.f;
-      if (scaled) {
-        __syncwarp();   // the previous tile's reads are done
-        for (int i = lane; i < p.bn; i += 32)
-          col_scale[i] = (b0 + i < p.rows_b) ? p.scale_b[b0 + i] : 0.f;
-        __syncwarp();
+      // The tile's column scales and the residual's first columns are requested while the k-loop
+      // runs: a lone tile per CTA pays for every load that waits for its accumulator.
+      if (scaled && p.coalesce) {
+        const long long c = b0 + 4 * (lane + 32 * half);
+        if (4 * (lane + 32 * half) < p.bn && c + 4 <= p.rows_b) {
+          float4 s;
+          asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w)
+                       : "l"(p.scale_b + c));
+        }
       }
+      // residual rows of the 64 columns from c0 on, four whole 128-byte lines an instruction
+      uint4 rq[8];
+      auto fetch_residual = [&](int c0) {
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const long long grow = (long long)tile_a * kBlockM + quad * 32 + it * 4 + (lane >> 3);
+          const int c = c0 + 8 * (lane & 7);
+          if (grow < p.rows_a && b0 + c + 8 <= p.rows_b && c + 8 <= p.bn)
+            rq[it] = *reinterpret_cast<const uint4*>(p.residual + grow * p.ldr + b0 + c);
+        }
+      };
+      const bool add_rows = p.coalesce && p.residual != nullptr;
+      if (add_rows && half * 64 < p.bn) fetch_residual(half * 64);
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 400 + acc, w)) break;
       tc_fence_after();
       const uint32_t t_addr =
@@ -399,13 +429,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (p.coalesce) {
         // 64 output columns at a time: each thread converts its row, the warp transposes
         // through its private staging tile, and every store instruction then writes four
-        // full 128-byte lines (rows) instead of 32 scattered 16-byte pieces.
-        uint8_t* stg = store_stage + (size_t)quad * kStoreStageBytes;
-        for (int c0 = 0; c0 < p.bn; c0 += 64) {
+        // full 128-byte lines (rows) instead of 32 scattered 16-byte pieces. The residual comes
+        // the same way in the other direction.
+        uint8_t* stg = store_stage + (size_t)(warp - 2) * kStoreStageBytes;
+        for (int c0 = half * 64; c0 < p.bn; c0 += 128) {
           uint32_t r0[32], r1[32];
           __syncwarp();
           tmem_ld_x32(t_addr + (uint32_t)c0, r0);
           tmem_ld_x32(t_addr + (uint32_t)(c0 + 32), r1);
+          if (add_rows) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it)
+              *reinterpret_cast<uint4*>(stg + stage_chunk(it * 4 + (lane >> 3), lane & 7)) = rq[it];
+            if (c0 + 128 < p.bn) fetch_residual(c0 + 128);
+            __syncwarp();
+          }
           tmem_ld_wait();
           const long long col = b0 + c0;
           if (row_ok) {
@@ -416,44 +454,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
               for (int t = 0; t < 8; ++t)
                 v[t] = __uint_as_float(j < 4 ? r0[8 * j + t] : r1[8 * (j - 4) + t]);
               const long long cj = col + 8 * j;
+              uint4* at = reinterpret_cast<uint4*>(stg + stage_chunk(lane, j));
               if (cj + 8 <= p.rows_b && c0 + 8 * j + 8 <= p.bn) {
                 if (scaled) {
-                  const float4 s0 = *reinterpret_cast<const float4*>(col_scale + c0 + 8 * j);
-                  const float4 s1 = *reinterpret_cast<const float4*>(col_scale + c0 + 8 * j + 4);
+                  const float4 s0 = *reinterpret_cast<const float4*>(p.scale_b + cj);
+                  const float4 s1 = *reinterpret_cast<const float4*>(p.scale_b + cj + 4);
                   v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
                   v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
                 }
-                if (p.bias != nullptr) {
-                  const uint4 q = *reinterpret_cast<const uint4*>(p.bias + cj);
-                  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-                  for (int u = 0; u < 4; ++u) {
-                    const float2 f = __bfloat1622float2(h[u]);
-                    v[2 * u] += f.x;
-                    v[2 * u + 1] += f.y;
-                  }
-                }
+                if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
                 if (p.act == 1) {
 #pragma unroll
                   for (int t = 0; t < 8; ++t) v[t] = gelu_erf(v[t]);
                 }
-                if (p.residual != nullptr) {
-                  const uint4 q = *reinterpret_cast<const uint4*>(p.residual + a_row * p.ldr + cj);
-                  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-                  for (int u = 0; u < 4; ++u) {
-                    const float2 f = __bfloat1622float2(h[u]);
-                    v[2 * u] += f.x;
-                    v[2 * u + 1] += f.y;
-                  }
-                }
+                if (add_rows) add8(v, *at);
               }
               uint4 q;
               q.x = pack_bf16x2(v[0], v[1]);
               q.y = pack_bf16x2(v[2], v[3]);
               q.z = pack_bf16x2(v[4], v[5]);
               q.w = pack_bf16x2(v[6], v[7]);
-              *reinterpret_cast<uint4*>(stg + lane * kStoreStagePitch + 16 * j) = q;
+              *at = q;
             }
           }
           __syncwarp();
@@ -469,13 +490,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const int rr = it * 4 + (lane >> 3);
             const long long grow = (long long)tile_a * kBlockM + quad * 32 + rr;
             if (grow < p.rows_a && col + 8 * ch + 8 <= p.rows_b && c0 + 8 * ch + 8 <= p.bn) {
-              const uint4 q = *reinterpret_cast<const uint4*>(stg + rr * kStoreStagePitch + 16 * ch);
+              const uint4 q = *reinterpret_cast<const uint4*>(stg + stage_chunk(rr, ch));
               *reinterpret_cast<uint4*>(base + (grow + row_off) * p.ldo + 8 * ch) = q;
             }
           }
         }
       } else
-      for (int c0 = 0; c0 < p.bn; c0 += 16) {
+      for (int c0 = half * 16; c0 < p.bn; c0 += 32) {
         uint32_t r[16];
         __syncwarp();
         tmem_ld_x16(t_addr + (uint32_t)c0, r);
@@ -504,7 +525,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         if (scaled) {
 #pragma unroll
-          for (int t = 0; t < 16; ++t) v[t] *= sa * col_scale[c0 + t];
+          for (int t = 0; t < 16; ++t)
+            v[t] *= sa * (b0 + c0 + t < p.rows_b ? p.scale_b[b0 + c0 + t] : 0.f);
         }
         if (!p.transposed) {
           const long long col = b0 + c0;
@@ -591,13 +613,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                 // on distinct banks
     const uint32_t my = cluster_ctarank();
     const int quad = warp & 3;
+    const int half = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
     // first barrier: every CTA of the cluster has consumed its last pipeline stage (its
     // epilogue warps arrive only after their accumulator is complete)
     cluster_sync();
     if (warp >= 2 && cluster_acc_ok) {
       const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-      for (int c0 = 0; c0 < p.bn; c0 += 16) {
+      for (int c0 = half * 16; c0 < p.bn; c0 += 32) {
         uint32_t r[16];
         __syncwarp();
         tmem_ld_x16(t_addr + (uint32_t)c0, r);
@@ -621,7 +644,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const long long col0 = (long long)tile_b * p.bn + (long long)my * cw;
       const float sa = (p.scale_a != nullptr && row_ok) ? p.scale_a[a_row] : 1.f;
       const float* slots = reinterpret_cast<const float*>(smem);
-      for (int j = 0; j < cw; j += 8) {
+      for (int j = half * 8; j < cw; j += 16) {
         float v[8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) v[t] = 0.f;
@@ -635,8 +658,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const long long col = col0 + j;
         if (!row_ok || col + 8 > p.rows_b) continue;
         if (p.scale_a != nullptr) {
-          const float4 s0 = *reinterpret_cast<const float4*>(col_scale + j);
-          const float4 s1 = *reinterpret_cast<const float4*>(col_scale + j + 4);
+          const float4 s0 = *reinterpret_cast<const float4*>(p.scale_b + col);
+          const float4 s1 = *reinterpret_cast<const float4*>(p.scale_b + col + 4);
           v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
           v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
         }
@@ -808,7 +831,7 @@ static int num_sms() {
 
 static int pick_stages(int bn) {
   const int stage_bytes = (int)kABytes + bn * kBlockK * 2;
-  int s = (227 * 1024 - 6144 - 4 * kStoreStageBytes) / stage_bytes;
+  int s = (227 * 1024 - 1024 - 256 - kStoreBytes) / stage_bytes;
   if (s > kMaxStages) s = kMaxStages;
   return s;
 }
@@ -1084,7 +1107,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   a.kblocks_per_split = (a.kblocks_total + a.splits - 1) / a.splits;
   a.splits = (a.kblocks_total + a.kblocks_per_split - 1) / a.kblocks_per_split;
   a.stages = pick_stages(a.bn);
-  a.tmem_cols = pow2_at_least(2u * (uint32_t)a.bn);
+  a.tmem_cols = pow2_at_least(2u * (uint32_t)(a.bn < 64 ? 64 : a.bn));  // (groups of 64 are read)
   if (a.cluster_splits > 1 &&
       (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) <
           (size_t)kBlockM * (a.bn + 4 * a.cluster_splits) * sizeof(float)) {
@@ -1148,7 +1171,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   const int total = a.tiles_a * a.tiles_b * a.splits;
   const int grid = (a.cluster_splits > 1 || total < sms) ? total : sms;
   const size_t smem =
-      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + 4 * kStoreStageBytes + 4096 + 1024;
+      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes + 1024;
   if (launch_pdl_cluster(gemm_bf16_kernel, dim3(grid), dim3(kGemmThreads), smem, stream,
                          a.cluster_splits > 1 ? (unsigned)a.cluster_splits : 1u, ta, tb,
                          a) != cudaSuccess)
@@ -1262,7 +1285,7 @@ int ab200_gemm_bf16_nn(const void* x, long long ldx, const void* wt, long long l
   a.tiles_a = (M + kBlockM - 1) / kBlockM;
   a.tiles_b = N / a.bn;
   a.stages = pick_stages(a.bn);
-  a.tmem_cols = pow2_at_least(2u * (uint32_t)a.bn);
+  a.tmem_cols = pow2_at_least(2u * (uint32_t)(a.bn < 64 ? 64 : a.bn));  // (groups of 64 are read)
   CUtensorMap ta, tb;
   if (get_tmap_bf16(&ta, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, kBlockM) != 0) return -4;
   if (make_tmap_2d(&tb, wt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (uint64_t)K, (uint64_t)N,
@@ -1272,7 +1295,7 @@ int ab200_gemm_bf16_nn(const void* x, long long ldx, const void* wt, long long l
   const int sms = num_sms();
   const int grid = total < sms ? total : sms;
   const size_t smem =
-      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + 4 * kStoreStageBytes + 4096 + 1024;
+      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes + 1024;
   gemm_bf16_kernel<<<grid, kGemmThreads, smem, stream>>>(ta, tb, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

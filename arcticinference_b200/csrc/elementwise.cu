@@ -238,6 +238,90 @@ layernorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
   }
 }
 
+// The same with one warp per row for rows of up to 1024 numbers (NV vectors of eight per lane), two
+// shuffle sums instead of four block barriers, gamma and beta held in registers while a warp walks
+// its rows and the next row on its way meanwhile. Memory-bound: a block per row (96 of its 128
+// threads with a vector of a 768-wide row, all idle at the barriers) took 62 us for the 50 MB of
+// 16384 such rows, this way 12 us.
+template <int NV>
+__global__ void __launch_bounds__(kNormThreads)
+layernorm_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
+                      const bf16* __restrict__ gamma, const bf16* __restrict__ beta,
+                      bf16* __restrict__ y, long long rows, int hidden, float eps) {
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int nvec = hidden / 8;
+  const long long step = (long long)gridDim.x * (kNormThreads / 32);
+  long long row = (long long)blockIdx.x * (kNormThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  uint4 g[NV], b[NV], in[NV], res[NV];
+  auto fetch = [&](long long r) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + 32 * j;
+      in[j] = res[j] = make_uint4(0, 0, 0, 0);
+      if (i < nvec) {
+        in[j] = reinterpret_cast<const uint4*>(x + r * (long long)hidden)[i];
+        if (residual) res[j] = reinterpret_cast<const uint4*>(residual + r * (long long)hidden)[i];
+      }
+    }
+  };
+  fetch(row);
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int i = lane + 32 * j;
+    g[j] = b[j] = make_uint4(0, 0, 0, 0);
+    if (i < nvec) {
+      g[j] = reinterpret_cast<const uint4*>(gamma)[i];
+      b[j] = reinterpret_cast<const uint4*>(beta)[i];
+    }
+  }
+  const float inv_n = 1.f / (float)hidden;
+  for (; row < rows; row += step) {
+    float vals[NV][8];
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      unpack8(in[j], vals[j]);
+      if (residual) {
+        float r[8];
+        unpack8(res[j], r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) vals[j][k] += r[k];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s += vals[j][k];
+    }
+    if (row + step < rows) fetch(row + step);
+    const float mean = warp_sum(s) * inv_n;
+    float v = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      if (lane + 32 * j < nvec) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float d = vals[j][k] - mean;
+          v += d * d;
+        }
+      }
+    }
+    const float inv = rsqrtf(warp_sum(v) * inv_n + eps);
+    uint4* yr = reinterpret_cast<uint4*>(y + row * (long long)hidden);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int i = lane + 32 * j;
+      if (i >= nvec) continue;
+      float gf[8], bf[8];
+      unpack8(g[j], gf);
+      unpack8(b[j], bf);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) vals[j][k] = (vals[j][k] - mean) * inv * gf[k] + bf[k];
+      yr[i] = pack8(vals[j]);
+    }
+  }
+}
+
 // -------------------------------- SiLU * mul --------------------------------
 // x: [T, nblk * 2 * inter] laid out as nblk blocks of (gate | up); out: [T, nblk * inter].
 // nblk = 1 is the usual fused gate/up layout; nblk > 1 is the rank-major layout whose
@@ -529,10 +613,26 @@ int ab200_layernorm(const void* x, const void* residual, const void* gamma, cons
                     void* y, long long T, int hidden, float eps, cudaStream_t stream) {
   if (T <= 0) return 0;
   if ((hidden % 8) || hidden > kNormThreads * kMaxVec * 8) return -2;
-  (void)launch_pdl(layernorm_kernel, dim3((unsigned)T), dim3(kNormThreads), 0, stream, 
-      reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(residual),
-      reinterpret_cast<const bf16*>(gamma), reinterpret_cast<const bf16*>(beta),
-      reinterpret_cast<bf16*>(y), hidden, eps);
+  const bf16* xb = reinterpret_cast<const bf16*>(x);
+  const bf16* rb = reinterpret_cast<const bf16*>(residual);
+  const bf16* gb = reinterpret_cast<const bf16*>(gamma);
+  const bf16* bb = reinterpret_cast<const bf16*>(beta);
+  bf16* yb = reinterpret_cast<bf16*>(y);
+  if (hidden <= 1024) {
+    // (a wider row no longer fits a warp's registers beside its successor)
+    const int rows_per_block = kNormThreads / 32;
+    const long long want = (T + rows_per_block - 1) / rows_per_block;
+    const dim3 grid((unsigned)(want < 148 * 8 ? want : 148 * 8));
+    switch ((hidden + 255) / 256) {
+      case 1: (void)launch_pdl(layernorm_warp_kernel<1>, grid, dim3(kNormThreads), 0, stream, xb, rb, gb, bb, yb, T, hidden, eps); break;
+      case 2: (void)launch_pdl(layernorm_warp_kernel<2>, grid, dim3(kNormThreads), 0, stream, xb, rb, gb, bb, yb, T, hidden, eps); break;
+      case 3: (void)launch_pdl(layernorm_warp_kernel<3>, grid, dim3(kNormThreads), 0, stream, xb, rb, gb, bb, yb, T, hidden, eps); break;
+      default: (void)launch_pdl(layernorm_warp_kernel<4>, grid, dim3(kNormThreads), 0, stream, xb, rb, gb, bb, yb, T, hidden, eps); break;
+    }
+  } else {
+    (void)launch_pdl(layernorm_kernel, dim3((unsigned)T), dim3(kNormThreads), 0, stream, xb, rb, gb,
+                     bb, yb, hidden, eps);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

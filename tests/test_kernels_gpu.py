@@ -56,6 +56,19 @@ def test_layernorm(T, H):
            3e-2, 2e-2)
 
 
+# one warp per row up to 1024 wide: part of a vector row, every vector count, more rows than warps
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 264), (5, 520), (4800, 768), (9481, 1016), (2, 1032)])
+def test_layernorm_rows(T, H):
+    x, r, g, b = _rand(T, H), _rand(T, H), _rand(H), _rand(H)
+    for res in (None, r):
+        v = x.double() if res is None else x.double() + res.double()
+        y = torch.nn.functional.layer_norm(v, (H,), g.double(), b.double(), 1e-12)
+        # one rounding to bf16, whose eight bits of significand put half a unit in the last place at up
+        # to 2^-8 of the value, and fp32 sums before it
+        bound = y.abs() * 2.0 ** -8 + 1e-5 * (1 + v.abs().amax(-1, keepdim=True))
+        assert ((ops.layernorm(x, g, b, 1e-12, residual=res).double() - y).abs() <= bound).all()
+
+
 def test_silu_mul():
     x = _rand(19, 2 * 14336)
     _close(ops.silu_mul(x), ref.silu_mul(x), 2e-2, 2e-2)

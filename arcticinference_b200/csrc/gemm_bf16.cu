@@ -121,6 +121,106 @@ __device__ __forceinline__ float gelu_erf(float x) {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
 
+// The epilogue of a tile whose output leaves in whole lines, one of eight warps: 32 rows from
+// warp_row0 on, alternate groups of 64 columns of the tile that starts at column b0.
+struct CoalescedTile {
+  uint4 rq[8];
+
+  // residual rows of the 64 columns from c0 on, four whole 128-byte lines an instruction
+  __device__ __forceinline__ void fetch_residual(const GemmArgs& p, long long warp_row0, long long b0,
+                                                 int c0, int lane) {
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const long long grow = warp_row0 + it * 4 + (lane >> 3);
+      const int c = c0 + 8 * (lane & 7);
+      if (grow < p.rows_a && b0 + c + 8 <= p.rows_b && c + 8 <= p.bn)
+        rq[it] = *reinterpret_cast<const uint4*>(p.residual + grow * p.ldr + b0 + c);
+    }
+  }
+
+  // before the accumulator is complete
+  __device__ __forceinline__ void prefetch(const GemmArgs& p, long long warp_row0, long long b0, int half,
+                                           int lane) {
+    if (p.residual != nullptr && half * 64 < p.bn) fetch_residual(p, warp_row0, b0, half * 64, lane);
+  }
+
+  // t_addr: the warp's lane quadrant of the accumulator; stg: its staging tile
+  __device__ __forceinline__ void store(const GemmArgs& p, uint32_t t_addr, uint8_t* stg,
+                                        long long warp_row0, long long b0, int half, int lane, float sa) {
+    const bool scaled = p.scale_a != nullptr;
+    const bool add_rows = p.residual != nullptr;
+    const bool row_ok = warp_row0 + lane < p.rows_a;
+    // 64 output columns at a time: each thread converts its row, the warp transposes
+    // through its private staging tile, and every store instruction then writes four
+    // full 128-byte lines (rows) instead of 32 scattered 16-byte pieces. The residual comes
+    // the same way in the other direction.
+    for (int c0 = half * 64; c0 < p.bn; c0 += 128) {
+      uint32_t r0[32], r1[32];
+      __syncwarp();
+      tmem_ld_x32(t_addr + (uint32_t)c0, r0);
+      tmem_ld_x32(t_addr + (uint32_t)(c0 + 32), r1);
+      if (add_rows) {
+#pragma unroll
+        for (int it = 0; it < 8; ++it)
+          *reinterpret_cast<uint4*>(stg + stage_chunk(it * 4 + (lane >> 3), lane & 7)) = rq[it];
+        if (c0 + 128 < p.bn) fetch_residual(p, warp_row0, b0, c0 + 128, lane);
+        __syncwarp();
+      }
+      tmem_ld_wait_dep(r0);
+      tmem_ld_wait_dep(r1);
+      const long long col = b0 + c0;
+      if (row_ok) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float v[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t)
+            v[t] = __uint_as_float(j < 4 ? r0[8 * j + t] : r1[8 * (j - 4) + t]);
+          const long long cj = col + 8 * j;
+          uint4* at = reinterpret_cast<uint4*>(stg + stage_chunk(lane, j));
+          if (cj + 8 <= p.rows_b && c0 + 8 * j + 8 <= p.bn) {
+            if (scaled) {
+              const float4 s0 = *reinterpret_cast<const float4*>(p.scale_b + cj);
+              const float4 s1 = *reinterpret_cast<const float4*>(p.scale_b + cj + 4);
+              v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
+              v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
+            }
+            if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
+            if (p.act == 1) {
+#pragma unroll
+              for (int t = 0; t < 8; ++t) v[t] = gelu_erf(v[t]);
+            }
+            if (add_rows) add8(v, *at);
+          }
+          uint4 q;
+          q.x = pack_bf16x2(v[0], v[1]);
+          q.y = pack_bf16x2(v[2], v[3]);
+          q.z = pack_bf16x2(v[4], v[5]);
+          q.w = pack_bf16x2(v[6], v[7]);
+          *at = q;
+        }
+      }
+      __syncwarp();
+      __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.out) + col;
+      long long row_off = 0;
+      if (p.peer_cols > 0) {  // a 64-column group never straddles a destination
+        base = p.peer_out[col / p.peer_cols] + col % p.peer_cols;
+        row_off = p.peer_row_off;
+      }
+      const int ch = lane & 7;
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int rr = it * 4 + (lane >> 3);
+        const long long grow = warp_row0 + rr;
+        if (grow < p.rows_a && col + 8 * ch + 8 <= p.rows_b && c0 + 8 * ch + 8 <= p.bn) {
+          const uint4 q = *reinterpret_cast<const uint4*>(stg + stage_chunk(rr, ch));
+          *reinterpret_cast<uint4*>(base + (grow + row_off) * p.ldo + 8 * ch) = q;
+        }
+      }
+    }
+  }
+};
+
 // Work item -> (A tile, B tile, K split). Cluster launches hold one item per CTA, the K splits
 // of a tile being the consecutive CTAs of one cluster.
 __device__ __forceinline__ void decode_work(const GemmArgs& p, int w, int& tile_a, int& tile_b,
@@ -408,93 +508,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                        : "l"(p.scale_b + c));
         }
       }
-      // residual rows of the 64 columns from c0 on, four whole 128-byte lines an instruction
-      uint4 rq[8];
-      auto fetch_residual = [&](int c0) {
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const long long grow = (long long)tile_a * kBlockM + quad * 32 + it * 4 + (lane >> 3);
-          const int c = c0 + 8 * (lane & 7);
-          if (grow < p.rows_a && b0 + c + 8 <= p.rows_b && c + 8 <= p.bn)
-            rq[it] = *reinterpret_cast<const uint4*>(p.residual + grow * p.ldr + b0 + c);
-        }
-      };
-      const bool add_rows = p.coalesce && p.residual != nullptr;
-      if (add_rows && half * 64 < p.bn) fetch_residual(half * 64);
+      const long long warp_row0 = (long long)tile_a * kBlockM + quad * 32;
+      CoalescedTile ct;
+      if (p.coalesce) ct.prefetch(p, warp_row0, b0, half, lane);
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 400 + acc, w)) break;
       tc_fence_after();
       const uint32_t t_addr =
           tmem_base + (uint32_t)acc * acc_stride + ((uint32_t)(quad * 32) << 16);
 
       if (p.coalesce) {
-        // 64 output columns at a time: each thread converts its row, the warp transposes
-        // through its private staging tile, and every store instruction then writes four
-        // full 128-byte lines (rows) instead of 32 scattered 16-byte pieces. The residual comes
-        // the same way in the other direction.
-        uint8_t* stg = store_stage + (size_t)(warp - 2) * kStoreStageBytes;
-        for (int c0 = half * 64; c0 < p.bn; c0 += 128) {
-          uint32_t r0[32], r1[32];
-          __syncwarp();
-          tmem_ld_x32(t_addr + (uint32_t)c0, r0);
-          tmem_ld_x32(t_addr + (uint32_t)(c0 + 32), r1);
-          if (add_rows) {
-#pragma unroll
-            for (int it = 0; it < 8; ++it)
-              *reinterpret_cast<uint4*>(stg + stage_chunk(it * 4 + (lane >> 3), lane & 7)) = rq[it];
-            if (c0 + 128 < p.bn) fetch_residual(c0 + 128);
-            __syncwarp();
-          }
-          tmem_ld_wait();
-          const long long col = b0 + c0;
-          if (row_ok) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float v[8];
-#pragma unroll
-              for (int t = 0; t < 8; ++t)
-                v[t] = __uint_as_float(j < 4 ? r0[8 * j + t] : r1[8 * (j - 4) + t]);
-              const long long cj = col + 8 * j;
-              uint4* at = reinterpret_cast<uint4*>(stg + stage_chunk(lane, j));
-              if (cj + 8 <= p.rows_b && c0 + 8 * j + 8 <= p.bn) {
-                if (scaled) {
-                  const float4 s0 = *reinterpret_cast<const float4*>(p.scale_b + cj);
-                  const float4 s1 = *reinterpret_cast<const float4*>(p.scale_b + cj + 4);
-                  v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
-                  v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
-                }
-                if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
-                if (p.act == 1) {
-#pragma unroll
-                  for (int t = 0; t < 8; ++t) v[t] = gelu_erf(v[t]);
-                }
-                if (add_rows) add8(v, *at);
-              }
-              uint4 q;
-              q.x = pack_bf16x2(v[0], v[1]);
-              q.y = pack_bf16x2(v[2], v[3]);
-              q.z = pack_bf16x2(v[4], v[5]);
-              q.w = pack_bf16x2(v[6], v[7]);
-              *at = q;
-            }
-          }
-          __syncwarp();
-          __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.out) + col;
-          long long row_off = 0;
-          if (p.peer_cols > 0) {  // a 64-column group never straddles a destination
-            base = p.peer_out[col / p.peer_cols] + col % p.peer_cols;
-            row_off = p.peer_row_off;
-          }
-          const int ch = lane & 7;
-#pragma unroll
-          for (int it = 0; it < 8; ++it) {
-            const int rr = it * 4 + (lane >> 3);
-            const long long grow = (long long)tile_a * kBlockM + quad * 32 + rr;
-            if (grow < p.rows_a && col + 8 * ch + 8 <= p.rows_b && c0 + 8 * ch + 8 <= p.bn) {
-              const uint4 q = *reinterpret_cast<const uint4*>(stg + stage_chunk(rr, ch));
-              *reinterpret_cast<uint4*>(base + (grow + row_off) * p.ldo + 8 * ch) = q;
-            }
-          }
-        }
+        ct.store(p, t_addr, store_stage + (size_t)(warp - 2) * kStoreStageBytes, warp_row0, b0, half,
+                 lane, sa);
       } else
       for (int c0 = half * 16; c0 < p.bn; c0 += 32) {
         uint32_t r[16];
@@ -710,6 +734,203 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 }
 
+// Two CTAs of a cluster on one tile of 256 rows by bn columns (cta_group::2), for products with more
+// rows than a few tiles: each CTA stages 128 rows of A and bn / 2 rows of B per k-block, the even
+// one issues the products for both, and each drains the 128 rows that its own TMEM holds.
+//
+// Why: one CTA with a 128 x 256 tile stages 48 KB per k-block of 512 tensor-core cycles and reads as
+// much again from shared memory for its operands, more than the 128 bytes a cycle that an SM's
+// shared memory moves. A pair needs 32 KB per CTA for the same work. 8192 x 28672 x 4096 bf16 went from
+// 1757 to 1219 us (1095 to 1578 TFLOP/s), fp8 from 866 to 678 us (2221 to 2837), 2048 x 28672 x 4096 from
+// 401 to 315 us, 16384 x 768 x 3072 + residual from 86 to 64 us. Tiles are walked in groups of eight rows of tiles, so
+// that the operands that the resident pairs share stay in L2.
+constexpr int kPairGroup = 8;
+
+__device__ __forceinline__ void decode_pair(const GemmArgs& p, int w, int& tile_a, int& tile_b) {
+  const int per_group = kPairGroup * p.tiles_b;
+  const int first = w / per_group * kPairGroup;
+  const int rows = min(kPairGroup, p.tiles_a - first);
+  const int r = w % per_group;
+  tile_a = first + r % rows;
+  tile_b = r / rows;
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
+                 const __grid_constant__ CUtensorMap tmap_b, const GemmArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  const uint32_t half_b = (uint32_t)p.bn / 2;
+  const uint32_t stage_bytes = kABytes + half_b * kBlockKBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)p.stages * stage_bytes);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint8_t* store_stage = reinterpret_cast<uint8_t*>(bars) + 256;
+  const uint32_t smem_base = smem_u32(smem);
+  const uint32_t bars_base = smem_u32(bars);
+  auto full_bar = [&](int s) { return bars_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bars_base + 8u * (kMaxStages + s); };
+  auto tfull_bar = [&](int a) { return bars_base + 8u * (2 * kMaxStages + a); };
+  auto tempty_bar = [&](int a) { return bars_base + 8u * (2 * kMaxStages + 2 + a); };
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank();
+
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(tfull_bar(a), 1);
+      mbar_init(tempty_bar(a), 2 * kEpilogueWarps);   // (the even CTA's: both CTAs drain)
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+    prefetch_tensormap(&tmap_a);
+    prefetch_tensormap(&tmap_b);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(tmem_slot), 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // the other CTA's barriers are ready for this one's copies and arrivals
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int total_work = p.tiles_a * p.tiles_b;
+  const int first_work = (int)blockIdx.x / 2, work_step = (int)gridDim.x / 2;
+
+  if (warp == 0) {
+    pdl_wait();
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int w = first_work; w < total_work && ok; w += work_step) {
+        int tile_a, tile_b;
+        decode_pair(p, w, tile_a, tile_b);
+        const int row_a = (2 * tile_a + rank) * kBlockM;
+        const int row_b = tile_b * p.bn + rank * (int)half_b;
+        for (int kb = 0; kb < p.kblocks_total; ++kb) {
+          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, 100 + stage, kb)) {
+            ok = false;
+            break;
+          }
+          // one barrier, the even CTA's, collects the four boxes of both CTAs
+          if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * stage_bytes);
+          const uint32_t full = map_to_cta(full_bar(stage), 0);
+          const uint32_t dst = smem_base + (uint32_t)stage * stage_bytes;
+          tma_load_2d_pair(dst, &tmap_a, full, kb * p.kblock_elems, row_a);
+          tma_load_2d_pair(dst + kABytes, &tmap_b, full, kb * p.kblock_elems, row_b);
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if (!ok) {
+        // Unwinding: copies already issued, by either CTA, get a short time to land.
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 20000000ull) {
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      const uint32_t idesc = p.fp8 ? make_idesc(2 * kBlockM, (uint32_t)p.bn, 0, 0, 0, 0)
+                                   : make_idesc(2 * kBlockM, (uint32_t)p.bn, 1, 1, 0, 0);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint64_t a0 = make_desc_kmajor_sw128(smem_base);
+      const uint64_t b0 = make_desc_kmajor_sw128(smem_base + kABytes);
+      const uint64_t stage_step = stage_bytes / 16;
+      int stage = 0;
+      uint32_t phase = 0;
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      bool ok = true;
+      for (int w = first_work; w < total_work && ok; w += work_step) {
+        if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
+                                               200 + acc, w)))
+          break;
+        tc_fence_after();
+        const uint32_t d_tmem = tm + (uint32_t)acc * 256u;
+        for (int kb = 0; kb < p.kblocks_total; ++kb) {
+          if (!__all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag, p.status,
+                                                 300 + stage, kb))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint64_t a_desc = a0 + (uint64_t)stage * stage_step;
+          const uint64_t b_desc = b0 + (uint64_t)stage * stage_step;
+          if (elect_one()) {
+            if (p.fp8) {
+#pragma unroll
+              for (int k = 0; k < kBlockKBytes / 32; ++k)
+                umma_f8_ss_pair(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc,
+                                (kb > 0 || k > 0) ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int k = 0; k < kBlockK / kUmmaK; ++k)
+                umma_f16_ss_pair(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc,
+                                 (kb > 0 || k > 0) ? 1u : 0u);
+            }
+            tc_commit_pair(empty_bar(stage));
+            if (kb == p.kblocks_total - 1) tc_commit_pair(tfull_bar(acc));
+          }
+          __syncwarp();
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1u;
+      }
+    }
+  } else {
+    pdl_wait();
+    const int quad = warp & 3;
+    const int half = (warp - 2) >> 2;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int w = first_work; w < total_work; w += work_step) {
+      int tile_a, tile_b;
+      decode_pair(p, w, tile_a, tile_b);
+      const long long warp_row0 = (long long)(2 * tile_a + rank) * kBlockM + quad * 32;
+      const long long col0 = (long long)tile_b * p.bn;
+      const float sa =
+          (p.scale_a != nullptr && warp_row0 + lane < p.rows_a) ? p.scale_a[warp_row0 + lane] : 1.f;
+      CoalescedTile ct;
+      ct.prefetch(p, warp_row0, col0, half, lane);
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 400 + acc, w)))
+        break;
+      tc_fence_after();
+      ct.store(p, tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * 256u,
+               store_stage + (size_t)(warp - 2) * kStoreStageBytes, warp_row0, col0, half, lane, sa);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // neither CTA leaves while the other may still signal it
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
 // out[m,n] = sum_s partial[s][m,n] (+bias[n]) -> activation -> (+residual[m,n])
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits,
                                      long long partial_stride, int M, int N,
@@ -881,6 +1102,31 @@ static double plan_cost_us(int tiles, int splits, int kblocks, int capacity, boo
   return t;
 }
 
+// Cycles that an SM spends on one k-block of a 128 x bn tile: the tensor core's (2 per column), or
+// what its shared memory takes to receive and to read the operands (128 bytes a cycle).
+static double kblock_cycles(int bn, int staged_b_rows) {
+  const double mma = 2.0 * bn, smem = 2.0 * (kABytes + 128.0 * staged_b_rows) / 128.0;
+  return mma > smem ? mma : smem;
+}
+
+// Width of the tiles that a product of more than one row of tiles is cut into, for `units` CTAs or
+// pairs that work at a time: the one with the least time in whole waves.
+static int pick_tile_width(int tiles_a, int N, int kblocks, int units, bool pair, double* cycles) {
+  int best = 0;
+  for (int bn = 256; bn >= 128; bn -= 64) {
+    if (bn > 128 && bn > ((N + 63) / 64) * 64) continue;
+    if (!pair && bn == 192) continue;
+    const long long tiles = (long long)tiles_a * ((N + bn - 1) / bn);
+    const double t = (double)((tiles + units - 1) / units) *
+                     (kblocks * kblock_cycles(bn, pair ? bn / 2 : bn) + 1000.0);
+    if (best == 0 || t < *cycles) {
+      best = bn;
+      *cycles = t;
+    }
+  }
+  return best;
+}
+
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 32;
   while (p < v) p <<= 1;
@@ -958,6 +1204,8 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   if (!attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return -3;
     attr_set[dev] = true;
   }
@@ -1119,6 +1367,34 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
                (peer_cols == 0 || (peer_cols % 64 == 0 && a.bn % 64 == 0)) &&
                (reinterpret_cast<uintptr_t>(bias) % 16) == 0 &&
                (residual == nullptr || ldr % 8 == 0);
+
+  // More than one row of tiles: CTA pairs, unless the tiles of single CTAs fill the GPU better.
+  if (!a.transposed && a.tiles_a > 1 && M > 256 && N >= 128 && peer_cols == 0 && (sync == nullptr || (sync->wait_world == 0 && sync->sig_world == 0)) && !w_tiled &&
+      a.coalesce) {
+    double single = 0, paired = 0;
+    pick_tile_width(a.tiles_a, N, a.kblocks_total, sms, false, &single);
+    const int tiles_pair = (M + 2 * kBlockM - 1) / (2 * kBlockM);
+    const int bn = pick_tile_width(tiles_pair, N, a.kblocks_total, sms / 2, true, &paired);
+    if (paired <= single && cluster_capacity(2, 227 * 1024 - 1024) > 0) {
+      a.bn = bn;
+      a.tiles_a = tiles_pair;
+      a.tiles_b = (N + bn - 1) / bn;
+      const int stage_bytes = (int)kABytes + bn / 2 * kBlockKBytes;
+      a.stages = (227 * 1024 - 1024 - 256 - kStoreBytes) / stage_bytes;
+      if (a.stages > kMaxStages) a.stages = kMaxStages;
+      CUtensorMap ta, tb;
+      if (get_tmap(&ta, pa, (uint64_t)M, (uint64_t)K, (uint64_t)lda, kBlockM, fp8) != 0 ||
+          get_tmap(&tb, pb, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)(bn / 2), fp8) != 0)
+        return -4;
+      const long long tiles = (long long)a.tiles_a * a.tiles_b;
+      const unsigned pairs = (unsigned)(tiles < sms / 2 ? tiles : sms / 2);
+      const size_t smem = (size_t)a.stages * stage_bytes + 256 + kStoreBytes + 1024;
+      return launch_pdl_cluster(gemm_pair_kernel, dim3(2 * pairs), dim3(kGemmThreads), smem, stream, 2u,
+                                ta, tb, a) == cudaSuccess
+                 ? 0
+                 : -5;
+    }
+  }
 
   TailSignal sig;
   memset(&sig, 0, sizeof(sig));

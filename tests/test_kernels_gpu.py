@@ -232,6 +232,31 @@ def test_linear_epilogue(M):
     ops.check_status()
 
 
+def _check_linear(M, N, K, fp8):
+    """Bias, GELU and residual of ``ops.linear`` against 64 bits. The bound: one rounding to bf16
+    (2^-8 of the value) and fp32 sums over K of products of the size of the operands."""
+    x, w, b, r = _rand(M, K), _rand(N, K, scale=1.0 / math.sqrt(K)), _rand(N), _rand(M, N)
+    xs, ws = (ops.quant_fp8_row(x), quant.quantize_weight_fp8_row(w)) if fp8 else (x, w)
+    if fp8:
+        z = (xs.q.double() @ ws.codes().double().t()) * xs.scale.double()[:, None] * ws.scale.double()
+    else:
+        z = x.double() @ w.double().t()
+    for kw, y in (({}, z), ({"bias": b, "residual": r}, z + b.double() + r.double()),
+                  ({"bias": b, "act": "gelu"}, torch.nn.functional.gelu(z + b.double()))):
+        out = ops.linear(xs, ws, **kw)
+        ops.check_status()
+        assert ((out.double() - y).abs() <= y.abs() * 2.0 ** -8 + 2e-4).all(), kw
+
+
+# CTA pairs: ends of 256-row tiles, of each tile width and of the ring of stages, one tile, several
+# groups of rows of tiles, more tiles than pairs
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("M,N,K", [(257, 128, 64), (511, 2312, 80), (513, 264, 16), (700, 200, 768),
+                                   (2049, 776, 448), (4100, 4104, 144), (9000, 2304, 768)])
+def test_linear_pairs(M, N, K, fp8):
+    _check_linear(M, N, K, fp8)
+
+
 @pytest.mark.parametrize("splits", [1, 2, 4, 8])
 def test_linear_split_k(splits):
     M, N, K = 24, 1024, 4096

@@ -931,6 +931,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 }
 
+}  // namespace ab200
+
+#include "common/gemm_few.cuh"
+
+namespace ab200 {
+
 // out[m,n] = sum_s partial[s][m,n] (+bias[n]) -> activation -> (+residual[m,n])
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits,
                                      long long partial_stride, int M, int N,
@@ -982,9 +988,10 @@ struct TmapKey {
   uint64_t rows, cols, ld;
   uint32_t box_rows;  // bit 31 set: e4m3 bytes instead of bf16
   uint64_t tile_stride_n = 0;  // tiled fp8 weights: bytes between 16-row tiles (0: row-major)
+  uint32_t group = 0;  // k-blocks per box of a map [K / block][rows][block] (0: two dimensions)
   bool operator==(const TmapKey& o) const {
     return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld &&
-           box_rows == o.box_rows && tile_stride_n == o.tile_stride_n;
+           box_rows == o.box_rows && tile_stride_n == o.tile_stride_n && group == o.group;
   }
 };
 struct TmapKeyHash {
@@ -995,12 +1002,13 @@ struct TmapKeyHash {
     h ^= k.ld * 0x165667B19E3779F9ull + (h << 6) + (h >> 2);
     h ^= k.box_rows * 0x27D4EB2F165667C5ull + (h << 6) + (h >> 2);
     h ^= k.tile_stride_n * 0x9FB21C651E98DF25ull + (h << 6) + (h >> 2);
+    h ^= k.group * 0xD6E8FEB86659FD93ull + (h << 6) + (h >> 2);
     return h;
   }
 };
 
 static int get_tmap(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld,
-                    uint32_t box_rows, bool fp8, uint64_t tile_stride_n = 0);
+                    uint32_t box_rows, bool fp8, uint64_t tile_stride_n = 0, uint32_t group = 0);
 static int get_tmap_bf16(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols,
                          uint64_t ld, uint32_t box_rows) {
   return get_tmap(out, ptr, rows, cols, ld, box_rows, false);
@@ -1010,10 +1018,10 @@ static int get_tmap_bf16(CUtensorMap* out, const void* ptr, uint64_t rows, uint6
 // tile_stride_n the distance between 16-row tiles (views of a larger tiled matrix keep their
 // parent's strides). A box of box_rows rows is box_rows/16 contiguous 2 KB pieces.
 static int get_tmap(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld,
-                    uint32_t box_rows, bool fp8, uint64_t tile_stride_n) {
+                    uint32_t box_rows, bool fp8, uint64_t tile_stride_n, uint32_t group) {
   static std::mutex mu;
   static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-  TmapKey key{ptr, rows, cols, ld, box_rows | (fp8 ? 0x80000000u : 0u), tile_stride_n};
+  TmapKey key{ptr, rows, cols, ld, box_rows | (fp8 ? 0x80000000u : 0u), tile_stride_n, group};
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) {
@@ -1022,7 +1030,14 @@ static int get_tmap(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t c
   }
   CUtensorMap m;
   int rc;
-  if (tile_stride_n > 0) {
+  if (group > 0) {
+    const uint64_t elems = fp8 ? kBlockKFp8 : kBlockK, bytes = fp8 ? 1 : 2;
+    const uint64_t dims[3] = {elems, rows, cols / elems};
+    const uint64_t strides[2] = {ld * bytes, 128};
+    const uint32_t box[3] = {(uint32_t)elems, box_rows, group};
+    rc = make_tmap_nd(&m, ptr, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims,
+                      strides, box);
+  } else if (tile_stride_n > 0) {
     const uint64_t dims[4] = {128, 16, cols / 128, (rows + 15) / 16};
     const uint64_t strides[3] = {128, ld, tile_stride_n};
     const uint32_t box[4] = {128, 16, 1, box_rows / 16};
@@ -1206,8 +1221,58 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(gemm_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(gemm_few_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return -3;
     attr_set[dev] = true;
+  }
+
+  const bool alone = sync == nullptr || (sync->wait_world == 0 && sync->sig_world == 0);
+  if (M <= 256 && peer_cols == 0 && alone && force_splits == 0 &&
+      (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
+    const int elems = fp8 ? kBlockKFp8 : kBlockK;
+    const int kblocks = (K + elems - 1) / elems;
+    const FewPlan plan = plan_few(M, N, kblocks, K % elems == 0 ? 4 : 1, num_sms(), cluster_capacity);
+    if (plan.bn > 0) {
+      FewArgs f;
+      f.scale_x = scale_x;
+      f.scale_w = scale_w;
+      f.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+      f.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
+      f.out = reinterpret_cast<__nv_bfloat16*>(out);
+      f.status = status;
+      f.ldo = ldo;
+      f.ldr = ldr;
+      f.M = M;
+      f.N = N;
+      f.x_rows = (M + 7) / 8 * 8;
+      f.bn = plan.bn;
+      f.stages = plan.stages;
+      f.group = plan.group;
+      f.groups = (kblocks + plan.group - 1) / plan.group;
+      f.groups_per_split = (f.groups + plan.splits - 1) / plan.splits;
+      f.splits = plan.splits;
+      f.act = act;
+      f.w_tiled = w_tiled ? 1 : 0;
+      // (without programmatic launches no kernel runs beside this one)
+      f.w_static = (w_static || !pdl_enabled()) ? 1 : 0;
+      f.tmem_cols = pow2_at_least((uint32_t)plan.bn * (M > 128 ? 2u : 1u));
+      f.ragged = K % elems != 0 ? 1 : 0;
+      const uint32_t group = f.ragged ? 0 : (uint32_t)plan.group;
+      CUtensorMap tx, tw;
+      if (get_tmap(&tx, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, (uint32_t)f.x_rows, fp8, 0, group) != 0 ||
+          get_tmap(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)(w_tiled ? w_tile_stride_k : ldw),
+                   (uint32_t)plan.bn, fp8, w_tiled ? (uint64_t)w_tile_stride_n : 0, w_tiled ? 0 : group) != 0)
+        return -4;
+      const unsigned ctas = (unsigned)((N + plan.bn - 1) / plan.bn * plan.splits);
+      return launch_pdl_cluster(fp8 ? gemm_few_kernel<true> : gemm_few_kernel<false>, dim3(ctas),
+                                dim3(kFewThreads), plan.smem, stream, (unsigned)plan.splits, tx, tw,
+                                f) == cudaSuccess
+                 ? 0
+                 : -5;
+    }
   }
 
   GemmArgs a;
@@ -1369,7 +1434,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
                (residual == nullptr || ldr % 8 == 0);
 
   // More than one row of tiles: CTA pairs, unless the tiles of single CTAs fill the GPU better.
-  if (!a.transposed && a.tiles_a > 1 && M > 256 && N >= 128 && peer_cols == 0 && (sync == nullptr || (sync->wait_world == 0 && sync->sig_world == 0)) && !w_tiled &&
+  if (!a.transposed && a.tiles_a > 1 && M > 256 && N >= 128 && peer_cols == 0 && alone && !w_tiled &&
       a.coalesce) {
     double single = 0, paired = 0;
     pick_tile_width(a.tiles_a, N, a.kblocks_total, sms, false, &single);

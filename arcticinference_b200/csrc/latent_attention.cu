@@ -73,14 +73,6 @@ struct LatentExt {
 
 __device__ __forceinline__ void bar_softmax() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld_wait_dep16(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                 "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]),
-                 "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
 __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -406,7 +398,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
         for (int g = 0; g < NR / 16; ++g) tmem_ld_x16(ts + 16u * g, sr[g]);
 #pragma unroll
-        for (int g = 0; g < NR / 16; ++g) tmem_ld_wait_dep16(sr[g]);
+        for (int g = 0; g < NR / 16; ++g) tmem_ld_wait_dep(sr[g]);
         if (need_mask) {
 #pragma unroll
           for (int i = 0; i < NR; ++i) {
@@ -461,7 +453,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_q,
             uint32_t r[16];
             const uint32_t to = tO + (uint32_t)(rc * NR + 16 * g) + lane_off;
             tmem_ld_x16(to, r);
-            tmem_ld_wait_dep16(r);
+            tmem_ld_wait_dep(r);
 #pragma unroll
             for (int i = 0; i < 16; ++i)
               r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha_s[16 * g + i]);
@@ -543,7 +535,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_q,
           uint32_t r[16];
           if (n_tiles > 0) {
             tmem_ld_x16(tO + (uint32_t)(rc * NR + 16 * g) + lane_off, r);
-            tmem_ld_wait_dep16(r);
+            tmem_ld_wait_dep(r);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) r[i] = 0u;

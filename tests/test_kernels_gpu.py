@@ -248,6 +248,16 @@ def _check_linear(M, N, K, fp8):
         assert ((out.double() - y).abs() <= y.abs() * 2.0 ** -8 + 2e-4).all(), kw
 
 
+# few tokens: one and two accumulators, odd token counts, features that end inside a tile, K that ends
+# inside a block or fills less than one, K split over the CTAs of a cluster, more blocks than stages
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (1, 4096, 4096), (3, 136, 80), (7, 6144, 2048), (50, 768, 768),
+                                   (127, 2312, 1040), (128, 28672, 4096), (129, 264, 48), (200, 768, 3072),
+                                   (255, 4096, 14336), (256, 32000, 512)])
+def test_linear_few_tokens(M, N, K, fp8):
+    _check_linear(M, N, K, fp8)
+
+
 # CTA pairs: ends of 256-row tiles, of each tile width and of the ring of stages, one tile, several
 # groups of rows of tiles, more tiles than pairs
 @pytest.mark.parametrize("fp8", [False, True])

@@ -47,10 +47,7 @@ __device__ __forceinline__ void few_store8(const FewArgs& p, int m, int c, float
     v[4] *= sx * s1.x; v[5] *= sx * s1.y; v[6] *= sx * s1.z; v[7] *= sx * s1.w;
   }
   if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + c));
-  if (p.act == 1) {
-#pragma unroll
-    for (int t = 0; t < 8; ++t) v[t] = gelu_erf(v[t]);
-  }
+  if (p.act == 1) gelu8(v);
   if (p.residual != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.residual + m * p.ldr + c));
   uint4 q;
   q.x = pack_bf16x2(v[0], v[1]);
@@ -77,7 +74,7 @@ template <bool FP8>
 __global__ void __launch_bounds__(kFewThreads, 1)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                 const FewArgs p) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const uint32_t w_bytes = (uint32_t)(p.group * p.bn) * 128u, x_bytes = (uint32_t)(p.group * p.x_rows) * 128u;

@@ -51,7 +51,8 @@ constexpr uint32_t kABytes = kBlockM * kBlockK * 2;
 // Per-epilogue-warp staging tile for coalesced loads and stores: 32 rows x 64 bf16, the 16-byte
 // chunks of a row XORed with the row so that eight lanes hit distinct banks both ways.
 constexpr int kStoreStageBytes = 32 * 128;
-constexpr int kStoreBytes = kEpilogueWarps * kStoreStageBytes;
+constexpr int kColumnBytes = 64 * 4;   // a warp's column factors or biases
+constexpr int kStoreBytes = kEpilogueWarps * (kStoreStageBytes + kColumnBytes);
 
 struct GemmArgs {
   int rows_a, rows_b, K;
@@ -117,14 +118,63 @@ __device__ __forceinline__ void add8(float (&v)[8], const uint4& q) {
   }
 }
 
-__device__ __forceinline__ float gelu_erf(float x) {
-  return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
+// x * Phi(x) as max(x, 0) - |x| Phi(-|x|), with Phi(-a) = exp(-a^2 / 2) p(t), t = 1 / (1 + c a): the classic
+// form of the error function's tail (Hastings; Abramowitz and Stegun 7.1.26), here with a polynomial of
+// degree eight fitted to 4e-8 of the value over a <= 13. Two values at a time, for the packed fp32
+// instructions. Off by at most 1.2e-7 between -1 and 1 and by 8e-6 of the value down to -12; 1 + erf(x)
+// is off by 8e-8 and loses all of the value below -6. Eleven instructions a value, two of them of the
+// special-function unit; with erff the GELU was most of what its epilogue did (16384 x 3072 x 768: 134 us,
+// 98 with this and the column values through shared memory, see CoalescedTile).
+__device__ __forceinline__ float2 gelu_x2(float2 x) {
+  auto both = [](float c) { return make_float2(c, c); };
+  const float2 a = make_float2(fminf(fabsf(x.x), 13.f), fminf(fabsf(x.y), 13.f));
+  const float2 d = fma_x2(both(0.22627417f), a, both(1.f));
+  const float2 t = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+  float2 p = both(-8.967171199e-02f);
+  p = fma_x2(p, t, both(3.590103068e-01f));
+  p = fma_x2(p, t, both(-4.005597391e-01f));
+  p = fma_x2(p, t, both(4.219819970e-01f));
+  p = fma_x2(p, t, both(-1.055775834e-01f));
+  p = fma_x2(p, t, both(1.450507083e-01f));
+  p = fma_x2(p, t, both(7.816432667e-02f));
+  p = fma_x2(p, t, both(9.167208235e-02f));
+  p = fma_x2(p, t, both(-7.036817162e-05f));
+  // (a NaN stays one through the exponential)
+  const float2 e = mul_x2(mul_x2(x, x), both(-0.7213475204f));
+  p = mul_x2(p, make_float2(ex2_approx(e.x), ex2_approx(e.y)));
+  return fma_x2(make_float2(-a.x, -a.y), p, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+}
+__device__ __forceinline__ float gelu_erf(float x) { return gelu_x2(make_float2(x, x)).x; }
+__device__ __forceinline__ void gelu8(float (&v)[8]) {
+#pragma unroll
+  for (int t = 0; t < 8; t += 2) {
+    const float2 y = gelu_x2(make_float2(v[t], v[t + 1]));
+    v[t] = y.x;
+    v[t + 1] = y.y;
+  }
 }
 
 // The epilogue of a tile whose output leaves in whole lines, one of eight warps: 32 rows from
 // warp_row0 on, alternate groups of 64 columns of the tile that starts at column b0.
 struct CoalescedTile {
   uint4 rq[8];
+  // This lane's two of the group's 64 column factors or biases; they reach the other lanes through shared
+  // memory. A load per eight columns from global memory, behind stores that might alias it, took
+  // longer than the products of a 768-deep tile: 16384 x 2304 x 768 + bias 65.7 -> 55.9 us, 8192 x 4096 x
+  // 14336 fp8 366 -> 320.
+  float cv[2];
+
+  __device__ __forceinline__ void fetch_columns(const GemmArgs& p, long long b0, int c0, int lane) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long c = b0 + c0 + lane + 32 * h;
+      cv[h] = 0.f;
+      if (c < p.rows_b) {
+        if (p.scale_a != nullptr) cv[h] = p.scale_b[c];
+        else if (p.bias != nullptr) cv[h] = __bfloat162float(p.bias[c]);
+      }
+    }
+  }
 
   // residual rows of the 64 columns from c0 on, four whole 128-byte lines an instruction
   __device__ __forceinline__ void fetch_residual(const GemmArgs& p, long long warp_row0, long long b0,
@@ -141,11 +191,12 @@ struct CoalescedTile {
   // before the accumulator is complete
   __device__ __forceinline__ void prefetch(const GemmArgs& p, long long warp_row0, long long b0, int half,
                                            int lane) {
+    fetch_columns(p, b0, half * 64, lane);
     if (p.residual != nullptr && half * 64 < p.bn) fetch_residual(p, warp_row0, b0, half * 64, lane);
   }
 
-  // t_addr: the warp's lane quadrant of the accumulator; stg: its staging tile
-  __device__ __forceinline__ void store(const GemmArgs& p, uint32_t t_addr, uint8_t* stg,
+  // t_addr: the warp's lane quadrant of the accumulator; stg: its staging tile; cols: its 64 floats
+  __device__ __forceinline__ void store(const GemmArgs& p, uint32_t t_addr, uint8_t* stg, float* cols,
                                         long long warp_row0, long long b0, int half, int lane, float sa) {
     const bool scaled = p.scale_a != nullptr;
     const bool add_rows = p.residual != nullptr;
@@ -159,13 +210,16 @@ struct CoalescedTile {
       __syncwarp();
       tmem_ld_x32(t_addr + (uint32_t)c0, r0);
       tmem_ld_x32(t_addr + (uint32_t)(c0 + 32), r1);
+      cols[lane] = cv[0];
+      cols[lane + 32] = cv[1];
+      if (c0 + 128 < p.bn) fetch_columns(p, b0, c0 + 128, lane);
       if (add_rows) {
 #pragma unroll
         for (int it = 0; it < 8; ++it)
           *reinterpret_cast<uint4*>(stg + stage_chunk(it * 4 + (lane >> 3), lane & 7)) = rq[it];
         if (c0 + 128 < p.bn) fetch_residual(p, warp_row0, b0, c0 + 128, lane);
-        __syncwarp();
       }
+      __syncwarp();
       tmem_ld_wait_dep(r0);
       tmem_ld_wait_dep(r1);
       const long long col = b0 + c0;
@@ -179,17 +233,17 @@ struct CoalescedTile {
           const long long cj = col + 8 * j;
           uint4* at = reinterpret_cast<uint4*>(stg + stage_chunk(lane, j));
           if (cj + 8 <= p.rows_b && c0 + 8 * j + 8 <= p.bn) {
+            const float4 s0 = *reinterpret_cast<const float4*>(cols + 8 * j);
+            const float4 s1 = *reinterpret_cast<const float4*>(cols + 8 * j + 4);
             if (scaled) {
-              const float4 s0 = *reinterpret_cast<const float4*>(p.scale_b + cj);
-              const float4 s1 = *reinterpret_cast<const float4*>(p.scale_b + cj + 4);
               v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
               v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
+              if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
+            } else if (p.bias != nullptr) {
+              v[0] += s0.x; v[1] += s0.y; v[2] += s0.z; v[3] += s0.w;
+              v[4] += s1.x; v[5] += s1.y; v[6] += s1.z; v[7] += s1.w;
             }
-            if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
-            if (p.act == 1) {
-#pragma unroll
-              for (int t = 0; t < 8; ++t) v[t] = gelu_erf(v[t]);
-            }
+            if (p.act == 1) gelu8(v);
             if (add_rows) add8(v, *at);
           }
           uint4 q;
@@ -221,6 +275,10 @@ struct CoalescedTile {
   }
 };
 
+__device__ __forceinline__ float* column_values(uint8_t* store_stage, int warp) {
+  return reinterpret_cast<float*>(store_stage + (size_t)kEpilogueWarps * kStoreStageBytes) + (warp - 2) * 64;
+}
+
 // Work item -> (A tile, B tile, K split). Cluster launches hold one item per CTA, the K splits
 // of a tile being the consecutive CTAs of one cluster.
 __device__ __forceinline__ void decode_work(const GemmArgs& p, int w, int& tile_a, int& tile_b,
@@ -245,9 +303,12 @@ __device__ __forceinline__ void decode_work(const GemmArgs& p, int w, int& tile_
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b, const GemmArgs p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
+    return;
+  }
   const uint32_t b_bytes = (uint32_t)p.bn * kBlockK * 2;
   const uint32_t stage_bytes = kABytes + b_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)p.stages * stage_bytes);
@@ -497,17 +558,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const bool row_ok = a_row < p.rows_a;
       const long long b0 = (long long)tile_b * p.bn;
       const float sa = (scaled && row_ok) ? p.scale_a[a_row] : 1.f;
-      // The tile's column scales and the residual's first columns are requested while the k-loop
+      // The tile's column values and the residual's first columns are requested while the k-loop
       // runs: a lone tile per CTA pays for every load that waits for its accumulator.
-      if (scaled && p.coalesce) {
-        const long long c = b0 + 4 * (lane + 32 * half);
-        if (4 * (lane + 32 * half) < p.bn && c + 4 <= p.rows_b) {
-          float4 s;
-          asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w)
-                       : "l"(p.scale_b + c));
-        }
-      }
       const long long warp_row0 = (long long)tile_a * kBlockM + quad * 32;
       CoalescedTile ct;
       if (p.coalesce) ct.prefetch(p, warp_row0, b0, half, lane);
@@ -517,8 +569,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tmem_base + (uint32_t)acc * acc_stride + ((uint32_t)(quad * 32) << 16);
 
       if (p.coalesce) {
-        ct.store(p, t_addr, store_stage + (size_t)(warp - 2) * kStoreStageBytes, warp_row0, b0, half,
-                 lane, sa);
+        ct.store(p, t_addr, store_stage + (size_t)(warp - 2) * kStoreStageBytes,
+                 column_values(store_stage, warp), warp_row0, b0, half, lane, sa);
       } else
       for (int c0 = half * 16; c0 < p.bn; c0 += 32) {
         uint32_t r[16];
@@ -758,9 +810,12 @@ __device__ __forceinline__ void decode_pair(const GemmArgs& p, int w, int& tile_
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b, const GemmArgs p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
+    return;
+  }
   const uint32_t half_b = (uint32_t)p.bn / 2;
   const uint32_t stage_bytes = kABytes + half_b * kBlockKBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)p.stages * stage_bytes);
@@ -913,7 +968,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         break;
       tc_fence_after();
       ct.store(p, tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * 256u,
-               store_stage + (size_t)(warp - 2) * kStoreStageBytes, warp_row0, col0, half, lane, sa);
+               store_stage + (size_t)(warp - 2) * kStoreStageBytes, column_values(store_stage, warp), warp_row0,
+               col0, half, lane, sa);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
@@ -1067,7 +1123,7 @@ static int num_sms() {
 
 static int pick_stages(int bn) {
   const int stage_bytes = (int)kABytes + bn * kBlockK * 2;
-  int s = (227 * 1024 - 1024 - 256 - kStoreBytes) / stage_bytes;
+  int s = (227 * 1024 - 256 - kStoreBytes) / stage_bytes;
   if (s > kMaxStages) s = kMaxStages;
   return s;
 }
@@ -1445,7 +1501,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
       a.tiles_a = tiles_pair;
       a.tiles_b = (N + bn - 1) / bn;
       const int stage_bytes = (int)kABytes + bn / 2 * kBlockKBytes;
-      a.stages = (227 * 1024 - 1024 - 256 - kStoreBytes) / stage_bytes;
+      a.stages = (227 * 1024 - 256 - kStoreBytes) / stage_bytes;
       if (a.stages > kMaxStages) a.stages = kMaxStages;
       CUtensorMap ta, tb;
       if (get_tmap(&ta, pa, (uint64_t)M, (uint64_t)K, (uint64_t)lda, kBlockM, fp8) != 0 ||
@@ -1453,7 +1509,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
         return -4;
       const long long tiles = (long long)a.tiles_a * a.tiles_b;
       const unsigned pairs = (unsigned)(tiles < sms / 2 ? tiles : sms / 2);
-      const size_t smem = (size_t)a.stages * stage_bytes + 256 + kStoreBytes + 1024;
+      const size_t smem = (size_t)a.stages * stage_bytes + 256 + kStoreBytes;
       return launch_pdl_cluster(gemm_pair_kernel, dim3(2 * pairs), dim3(kGemmThreads), smem, stream, 2u,
                                 ta, tb, a) == cudaSuccess
                  ? 0
@@ -1512,7 +1568,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   const int total = a.tiles_a * a.tiles_b * a.splits;
   const int grid = (a.cluster_splits > 1 || total < sms) ? total : sms;
   const size_t smem =
-      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes + 1024;
+      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes;
   if (launch_pdl_cluster(gemm_bf16_kernel, dim3(grid), dim3(kGemmThreads), smem, stream,
                          a.cluster_splits > 1 ? (unsigned)a.cluster_splits : 1u, ta, tb,
                          a) != cudaSuccess)
@@ -1636,7 +1692,7 @@ int ab200_gemm_bf16_nn(const void* x, long long ldx, const void* wt, long long l
   const int sms = num_sms();
   const int grid = total < sms ? total : sms;
   const size_t smem =
-      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes + 1024;
+      (size_t)a.stages * (kABytes + (size_t)a.bn * kBlockK * 2) + 256 + kStoreBytes;
   gemm_bf16_kernel<<<grid, kGemmThreads, smem, stream>>>(ta, tb, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

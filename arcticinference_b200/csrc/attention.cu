@@ -738,6 +738,444 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   }
 }
 
+// Two 128-row tiles per CTA against the same keys and values (prefill and encoder calls with enough
+// rows): while four warps take one tile's softmax, the tensor core works on the other's products.
+// Why: with one tile a CTA waits for its softmax (3300 cycles per 128 x 128 tile at head dimension
+// 128, of which the tensor core needs 1024 and the exponentials as many). 8192 tokens behind 24576 cached
+// ones, 32 heads of 128: 4823 us with one tile, 3252 with two (798 -> 1183 TFLOP/s); 4 x 2048 tokens: 291 ->
+// 186; 32 texts of 512 tokens, 12 heads of 64: 122 -> 79.
+//
+// A thread owns a whole row of S, so no row value crosses a warp. P (bf16) goes back to tensor memory
+// over the columns of S it came from and is the A operand of P V from there, which leaves shared
+// memory to Q (64 KB) and two stages of K and V (128 KB), and tensor memory to two S and two O. The
+// products of a tile are issued P V(j), S(j + 1): in order, so S(j + 1) finds P(j) consumed, and once
+// S(j + 1) is complete O may be rescaled. O is rescaled only when a row's maximum has grown by more
+// than kRescaleLog2 in units of the base-2 exponential: until then the old reference point serves (P
+// and the row sum, which share it, stay below 2^8 times their usual size, in formats whose precision
+// does not depend on the size).
+constexpr float kRescaleLog2 = 8.f;
+constexpr int kWideKeys = 128;
+constexpr int kWideRows = 256;   // `tile_keys` of calls whose work items hold two tiles of rows
+constexpr int kWideThreads = 10 * 32;   // 2 x 4 softmax warps, TMA, MMA
+
+template <int D>
+__global__ void __launch_bounds__(kWideThreads, 1)
+attention_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                      const __grid_constant__ CUtensorMap tmap_v, const AttnArgs p) {
+  constexpr int TK = kWideKeys;
+  constexpr uint32_t kQBytes = 128 * D * 2;
+  constexpr uint32_t kKVBytes = TK * D * 2;
+  constexpr uint32_t kHalf = TK * 128;     // bytes of one 64-wide d half of a K/V stage
+  constexpr int kTmaWarp = 8, kMmaWarp = 9;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  const unsigned int total_blocks = gridDim.x;
+  pdl_trigger();
+  if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_wait();
+    if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
+    tail_signal(p.sig, total_blocks);
+    return;
+  }
+  const uint32_t sQ = smem_u32(smem);           // 2 tiles
+  const uint32_t sK = sQ + 2 * kQBytes;         // 2 stages
+  const uint32_t sV = sK + 2 * kKVBytes;        // 2 stages
+  uint8_t* pV = smem + 2 * kQBytes + 2 * kKVBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pV + 2 * kKVBytes);
+  const uint32_t bb = smem_u32(bars);
+  const uint32_t q_full = bb;
+  auto k_full = [&](int s) { return bb + 8u * (1 + s); };
+  auto k_empty = [&](int s) { return bb + 8u * (3 + s); };
+  auto v_full = [&](int s) { return bb + 8u * (5 + s); };
+  auto v_empty = [&](int s) { return bb + 8u * (7 + s); };
+  auto s_full = [&](int t) { return bb + 8u * (9 + t); };
+  auto p_full = [&](int t) { return bb + 8u * (11 + t); };
+  auto o_full = [&](int t) { return bb + 8u * (13 + t); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int* wk = p.work + (long long)(blockIdx.x / p.Hkv) * 8;
+  const int seq = wk[0];
+  const int q_tok0 = wk[1];
+  const int n_q_tok = wk[2];
+  if (n_q_tok <= 0) {  // padding entry of a fixed-size work list
+    pdl_wait();
+    tail_signal(p.sig, total_blocks);
+    return;
+  }
+  const int q_pos0 = wk[3];
+  const int kv_start = wk[4];
+  int kv_end = wk[5];
+  const int split = wk[6];
+  const int num_splits = wk[7];
+  const int kvh = blockIdx.x % p.Hkv;
+  const int tile_tok = 128 / p.G;    // tokens of a 128-row tile
+  if (p.causal) kv_end = min(kv_end, q_pos0 + n_q_tok);
+  // tiles of keys that the rows of tile t see
+  auto tiles_of = [&](int t) -> int {
+    const int toks = min(n_q_tok - t * tile_tok, tile_tok);
+    if (toks <= 0) return 0;
+    const int end = p.causal ? min(kv_end, q_pos0 + t * tile_tok + toks) : kv_end;
+    return end > kv_start ? (end - kv_start + TK - 1) / TK : 0;
+  };
+  const int n0 = tiles_of(0), n1 = tiles_of(1);
+  const int n_tiles = max(n0, n1);
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(k_full(s), 1);
+      mbar_init(k_empty(s), 1);
+      mbar_init(v_full(s), 1);
+      mbar_init(v_empty(s), 1);
+      mbar_init(s_full(s), 1);
+      mbar_init(p_full(s), 4);
+      mbar_init(o_full(s), 1);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+    prefetch_tensormap(&tmap_q);
+    prefetch_tensormap(&tmap_k);
+    prefetch_tensormap(&tmap_v);
+  }
+  if (warp == kMmaWarp) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  // Values that are never loaded (the last tile's, past the sequence's last block) meet P = 0 and
+  // must be finite; a stage that an earlier tile has filled is.
+  if (p.block_size > 0 && (n_tiles == 1 || n_tiles == 2)) {
+    const int last = kv_end - kv_start - (n_tiles - 1) * TK;
+    const int r_first = (last + p.block_size - 1) / p.block_size * p.block_size;
+    const int vecs = (TK - r_first) * 8;
+#pragma unroll
+    for (int h = 0; h < D / 64; ++h) {
+      uint4* z = reinterpret_cast<uint4*>(pV + (n_tiles - 1) * kKVBytes + h * kHalf + r_first * 128);
+      for (int i = threadIdx.x; i < vecs; i += kWideThreads) z[i] = make_uint4(0, 0, 0, 0);
+    }
+  }
+  fence_proxy_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  const uint32_t tmem_base = *tmem_slot;
+  // S (and P over it) of tile t at columns 128 t, O at 256 + D t
+
+  if (warp == kTmaWarp) {
+    if (lane == 0 && n_tiles > 0) {
+      const int tiles = n1 > 0 ? 2 : 1;
+      mbar_arrive_expect_tx(q_full, (uint32_t)tiles * kQBytes);
+      for (int t = 0; t < tiles; ++t)
+        for (int h = 0; h < D / 64; ++h)
+          tma_load_4d(sQ + (uint32_t)t * kQBytes + h * 16384u, &tmap_q, q_full, h * 64, 0, kvh,
+                      q_tok0 + t * tile_tok);
+    }
+    const int bs = p.block_size;
+    const int* bt = bs > 0 ? p.block_tables + (long long)seq * p.max_blocks : nullptr;
+    bool ok = true;
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int st = j & 1;
+      const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+      const int key0 = kv_start + j * TK;
+      const int nkeys = min(TK, kv_end - key0);
+      for (int kv = 0; kv < 2; ++kv) {
+        const uint32_t full = kv == 0 ? k_full(st) : v_full(st);
+        const uint32_t empty = kv == 0 ? k_empty(st) : v_empty(st);
+        const uint32_t dst = (kv == 0 ? sK : sV) + (uint32_t)st * kKVBytes;
+        const CUtensorMap* tm = kv == 0 ? &tmap_k : &tmap_v;
+        if (!mbar_wait(empty, ph ^ 1u, abort_flag, p.status, 500 + kv * 10 + st, j)) {
+          ok = false;
+          break;
+        }
+        if (bs > 0) {
+          const int nblk = (nkeys + bs - 1) / bs;
+          if (lane == 0) mbar_arrive_expect_tx(full, (uint32_t)(nblk * bs * (D / 64) * 128));
+          __syncwarp();
+          if (lane < nblk) {
+            const int bid = bt[key0 / bs + lane];
+            for (int h = 0; h < D / 64; ++h)
+              tma_load_4d(dst + h * kHalf + (uint32_t)(lane * bs) * 128u, tm, full, h * 64, 0, kvh,
+                          bid);
+          }
+        } else {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(full, kKVBytes);
+            for (int h = 0; h < D / 64; ++h)
+              tma_load_3d(dst + h * kHalf, tm, full, h * 64, kvh, seq + key0);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    if (n_tiles > 0) {
+      const uint32_t idesc_s = make_idesc(128, TK, 1, 1, 0, 0);
+      const uint32_t idesc_pv = make_idesc(128, D, 1, 1, 0, 1);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint64_t q_d = make_desc_kmajor_sw128(sQ), k_d = make_desc_kmajor_sw128(sK);
+      const uint64_t v_d = make_desc_mnmajor_sw128(sV, kHalf);
+      auto wait = [&](uint32_t bar, uint32_t parity, int code, int j) -> bool {
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.status, code, j));
+      };
+      // S of tile t against the keys of tile j
+      auto issue_s = [&](int t, int j) {
+        const uint64_t qd = q_d + (uint64_t)(t * (int)(kQBytes / 16));
+        const uint64_t kd = k_d + (uint64_t)((j & 1) * (int)(kKVBytes / 16));
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k)
+            umma_f16_ss(tm + (uint32_t)t * 128u, qd + (uint64_t)((k / 4) * 1024 + 2 * (k % 4)),
+                        kd + (uint64_t)((k / 4) * (int)(kHalf / 16) + 2 * (k % 4)), idesc_s,
+                        k > 0 ? 1u : 0u);
+          tc_commit(s_full(t));
+        }
+        __syncwarp();
+      };
+      auto issue_pv = [&](int t, int j, bool last) {
+        const uint64_t vd = v_d + (uint64_t)((j & 1) * (int)(kKVBytes / 16));
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < TK / 16; ++k)
+            umma_f16_ts(tm + 256u + (uint32_t)(t * D), tm + (uint32_t)t * 128u + 8u * k,
+                        vd + (uint64_t)(128 * k), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+          if (last) tc_commit(o_full(t));
+        }
+        __syncwarp();
+      };
+      auto release = [&](uint32_t bar) {
+        if (elect_one()) tc_commit(bar);
+        __syncwarp();
+      };
+      bool ok = wait(q_full, 0, 600, 0) && wait(k_full(0), 0, 610, 0);
+      if (ok) {
+        tc_fence_after();
+        if (n0 > 0) issue_s(0, 0);
+        if (n1 > 0) issue_s(1, 0);
+        release(k_empty(0));
+      }
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        ok = wait(v_full(j & 1), (uint32_t)(j >> 1) & 1u, 630, j);
+        if (ok && j + 1 < n_tiles) ok = wait(k_full((j + 1) & 1), (uint32_t)((j + 1) >> 1) & 1u, 611, j);
+#pragma unroll
+        for (int t = 0; t < 2 && ok; ++t) {
+          const int n = t == 0 ? n0 : n1;
+          if (j < n) {
+            ok = wait(p_full(t), (uint32_t)j & 1u, 640 + t, j);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t, j, j + 1 == n);
+            if (j + 1 < n) issue_s(t, j + 1);
+          }
+        }
+        if (ok) {
+          release(v_empty(j & 1));
+          if (j + 1 < n_tiles) release(k_empty((j + 1) & 1));
+        }
+      }
+    }
+  } else {
+    // ------------------------------ softmax warps ------------------------------
+    const int t = warp >> 2;            // tile
+    const int quad = warp & 3;          // TMEM lane quadrant this warp may read
+    const int row = quad * 32 + lane;
+    const int my_tiles = t == 0 ? n0 : n1;
+    const int tok_local = t * tile_tok + row / p.G;
+    const int g = row % p.G;
+    const bool valid_row = tok_local < n_q_tok && g < p.g_heads;
+    const int q_pos = q_pos0 + tok_local;
+    const int limit = p.causal ? min(q_pos, kv_end - 1) : kv_end - 1;  // last visible key
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const uint32_t ts = tmem_base + (uint32_t)t * 128u + lane_off;
+    const uint32_t to = tmem_base + 256u + (uint32_t)(t * D) + lane_off;
+    // rows of this warp that are all padding only keep the barrier protocol going
+    const bool warp_active = t * tile_tok + quad * 32 / p.G < n_q_tok;
+    const float sc = p.scale_log2;
+    float m = -INFINITY;    // reference point of the exponentials
+    float l = 0.f;
+    bool ok = true;
+    for (int j = 0; j < my_tiles && ok; ++j) {
+      if (!__all_sync(0xffffffffu, mbar_wait(s_full(t), (uint32_t)j & 1u, abort_flag, p.status, 700 + t, j))) {
+        ok = false;
+        break;
+      }
+      if (!warp_active) {
+        if (lane == 0) mbar_arrive(p_full(t));
+        continue;
+      }
+      tc_fence_after();
+      const int key0 = kv_start + j * TK;
+      const bool need_mask = __any_sync(0xffffffffu, key0 + TK - 1 > limit);
+      uint32_t ra[32], rb[32];
+      auto hide = [&](uint32_t (&r)[32], int c) {
+        const int last = limit - key0 - 32 * c;   // last visible column of the chunk
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i > last) r[i] = 0xff800000u;
+      };
+      // pass 1: row maximum
+      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+      tmem_ld_x32(ts, ra);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t(&cur)[32] = (c & 1) ? rb : ra;
+        uint32_t(&nxt)[32] = (c & 1) ? ra : rb;
+        tmem_ld_wait_dep(cur);
+        tmem_ld_x32(ts + (uint32_t)((c + 1) & 3) * 32u, nxt);   // (chunk 0 again for pass 2)
+        if (need_mask) hide(cur, c);
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          mx0 = fmaxf(fmaxf(mx0, __uint_as_float(cur[i])), __uint_as_float(cur[i + 1]));
+          mx1 = fmaxf(fmaxf(mx1, __uint_as_float(cur[i + 2])), __uint_as_float(cur[i + 3]));
+          mx2 = fmaxf(fmaxf(mx2, __uint_as_float(cur[i + 4])), __uint_as_float(cur[i + 5]));
+          mx3 = fmaxf(fmaxf(mx3, __uint_as_float(cur[i + 6])), __uint_as_float(cur[i + 7]));
+        }
+      }
+      const float m_tile = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+      // (a row that has seen no key yet holds O = 0 and l = 0: its reference point is free)
+      const bool grow = m != -INFINITY && (m_tile - m) * sc > kRescaleLog2;
+      if (m == -INFINITY) m = m_tile;
+      if (__any_sync(0xffffffffu, grow)) {
+        // S(j) is complete, so P V(j - 1), issued before it, is too
+        tmem_ld_wait_dep(ra);
+        const float alpha = grow ? ex2_approx((m - m_tile) * sc) : 1.f;
+        if (grow) m = m_tile;
+        l *= alpha;
+        uint32_t rc[32];
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          tmem_ld_x32(to + (uint32_t)c * 32u, rc);
+          tmem_ld_wait_dep(rc);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) rc[i] = __float_as_uint(__uint_as_float(rc[i]) * alpha);
+          tmem_st_x32(to + (uint32_t)c * 32u, rc);
+        }
+      }
+      const float neg = m == -INFINITY ? 0.f : -m * sc;
+      // pass 2: probabilities, over the columns of S that have been read
+      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+      const float2 sc2 = make_float2(sc, sc), neg2 = make_float2(neg, neg);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t(&cur)[32] = (c & 1) ? rb : ra;
+        uint32_t(&nxt)[32] = (c & 1) ? ra : rb;
+        tmem_ld_wait_dep(cur);
+        if (c < 3) tmem_ld_x32(ts + (uint32_t)(c + 1) * 32u, nxt);
+        if (need_mask) hide(cur, c);
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          const float2 x0 = fma_x2(make_float2(__uint_as_float(cur[i]), __uint_as_float(cur[i + 1])), sc2, neg2);
+          const float2 x1 = fma_x2(make_float2(__uint_as_float(cur[i + 2]), __uint_as_float(cur[i + 3])), sc2, neg2);
+          const float2 e0 = make_float2(ex2_approx(x0.x), ex2_approx(x0.y));
+          const float2 e1 = make_float2(ex2_approx(x1.x), ex2_approx(x1.y));
+          s0 = add_x2(s0, e0);
+          s1 = add_x2(s1, e1);
+          pk[i / 2] = pack_bf16x2(e0.x, e0.y);
+          pk[i / 2 + 1] = pack_bf16x2(e1.x, e1.y);
+        }
+        tmem_st_x16(ts + (uint32_t)c * 16u, pk);
+      }
+      l += (s0.x + s0.y) + (s1.x + s1.y);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full(t));
+    }
+    if (ok && my_tiles > 0 && warp_active) {
+      ok = __all_sync(0xffffffffu, mbar_wait(o_full(t), 0, abort_flag, p.status, 720, my_tiles));
+      tc_fence_after();
+    }
+    if (ok && warp_active) {  // warp-uniform: every lane takes part in the TMEM reads
+      const long long tok = (long long)q_tok0 + tok_local;
+      const int head = kvh * p.g_heads + g;
+      const float inv_l = l > 0.f ? 1.f / l : 0.f;
+      const float lse = l > 0.f ? m * p.scale + logf(l) : -INFINITY;
+      __nv_bfloat16* dst16 = p.out + tok * p.ldo + (long long)head * D;
+      if (p.peer_tokens > 0)
+        dst16 = p.peer_out[tok / p.peer_tokens] + (tok % p.peer_tokens) * p.ldo + (long long)head * D;
+      float* dst32 = p.o_part + (((long long)split * p.T + tok) * p.Hq + head) * D;
+      if (num_splits <= 1 && my_tiles > 0) {
+        // whole rows through this tile's Q, which its last product no longer needs
+        constexpr int kCh = D / 8;   // 16-byte chunks per row
+        uint8_t* tile = smem + (size_t)t * kQBytes;
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t rc[32];
+          tmem_ld_x32(to + (uint32_t)c * 32u, rc);
+          tmem_ld_wait_dep(rc);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int j = c * 4 + i;
+            uint4 q;
+            q.x = pack_bf16x2(__uint_as_float(rc[8 * i]) * inv_l, __uint_as_float(rc[8 * i + 1]) * inv_l);
+            q.y = pack_bf16x2(__uint_as_float(rc[8 * i + 2]) * inv_l, __uint_as_float(rc[8 * i + 3]) * inv_l);
+            q.z = pack_bf16x2(__uint_as_float(rc[8 * i + 4]) * inv_l, __uint_as_float(rc[8 * i + 5]) * inv_l);
+            q.w = pack_bf16x2(__uint_as_float(rc[8 * i + 6]) * inv_l, __uint_as_float(rc[8 * i + 7]) * inv_l);
+            *reinterpret_cast<uint4*>(tile + (size_t)row * 128 + (size_t)(j >> 3) * 16384 +
+                                      (((j & 7) ^ (row & 7)) * 16)) = q;
+          }
+        }
+        __syncwarp();
+        const unsigned long long my_dst = valid_row ? reinterpret_cast<unsigned long long>(dst16) : 0ull;
+        const int j = lane % kCh;
+#pragma unroll
+        for (int it = 0; it < kCh; ++it) {
+          const int rl = it * (32 / kCh) + lane / kCh;  // row of this quadrant
+          const int rr = quad * 32 + rl;
+          const unsigned long long d = __shfl_sync(0xffffffffu, my_dst, rl);
+          if (d != 0ull)
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(d) + 8 * j) =
+                *reinterpret_cast<const uint4*>(tile + (size_t)rr * 128 + (size_t)(j >> 3) * 16384 +
+                                                (((j & 7) ^ (rr & 7)) * 16));
+        }
+        if (valid_row && p.lse_out) p.lse_out[tok * p.Hq + head] = lse;
+      } else {
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t rc[32];
+          if (my_tiles > 0) {
+            tmem_ld_x32(to + (uint32_t)c * 32u, rc);
+            tmem_ld_wait_dep(rc);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) rc[i] = 0u;
+          }
+          if (valid_row) {
+            if (num_splits <= 1) {
+#pragma unroll
+              for (int i = 0; i < 32; i += 8)
+                *reinterpret_cast<uint4*>(dst16 + c * 32 + i) = make_uint4(0, 0, 0, 0);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(dst32 + c * 32 + i) = make_float4(
+                    __uint_as_float(rc[i]) * inv_l, __uint_as_float(rc[i + 1]) * inv_l,
+                    __uint_as_float(rc[i + 2]) * inv_l, __uint_as_float(rc[i + 3]) * inv_l);
+            }
+          }
+        }
+        if (valid_row) {
+          if (num_splits > 1)
+            p.lse_part[((long long)split * p.T + tok) * p.Hq + head] = lse;
+          else if (p.lse_out)
+            p.lse_out[tok * p.Hq + head] = lse;
+        }
+      }
+    }
+  }
+
+  tail_signal(p.sig, total_blocks);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 // Fold split-KV partials: out = sum_s w_s O_s / sum_s w_s, w_s = exp(lse_s - max lse).
 // tok_splits[t] = number of splits that cover token t (<= 1: nothing to do).
 template <int D, bool EXT>
@@ -814,7 +1252,22 @@ struct AttnExt {
   float softcap;
 };
 
-template <int DK, int D, int TK, bool EXT, bool CAP = false>
+// The kernel, its block and its shared memory; WIDE: two tiles of rows per CTA.
+template <int DK, int D, int TK, bool EXT, bool CAP, bool WIDE>
+struct AttnLaunch {
+  static constexpr int kThreads = AttnShape<DK, TK>::kThreads;
+  static constexpr size_t kSmem = 128 * DK * 2 + 2 * (size_t)TK * (DK + D) * 2 +
+                                  (AttnShape<DK, TK>::kPrefill ? 2 : 1) * (size_t)128 * TK * 2 + 256;
+  static auto kernel() { return attention_kernel<DK, D, TK, EXT, CAP>; }
+};
+template <int DK, int D, int TK, bool EXT, bool CAP>
+struct AttnLaunch<DK, D, TK, EXT, CAP, true> {
+  static constexpr int kThreads = kWideThreads;
+  static constexpr size_t kSmem = 2 * 128 * D * 2 + 4 * (size_t)kWideKeys * D * 2 + 256;
+  static auto kernel() { return attention_wide_kernel<D>; }
+};
+
+template <int DK, int D, int TK, bool EXT, bool CAP = false, bool WIDE = false>
 static int launch_attention(const void* q, long long ldq, const void* k, const void* v,
                             long long ld_kv, long long num_blocks, int block_size,
                             const int* block_tables, int max_blocks, const int* work, int num_work,
@@ -835,11 +1288,10 @@ static int launch_attention(const void* q, long long ldq, const void* k, const v
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -3;
-  const size_t smem =
-      128 * DK * 2 + 2 * (size_t)TK * (DK + D) * 2 +
-      (AttnShape<DK, TK>::kPrefill ? 2 : 1) * (size_t)128 * TK * 2 + 256;
+  using L = AttnLaunch<DK, D, TK, EXT, CAP, WIDE>;
+  const size_t smem = L::kSmem;
   if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(attention_kernel<DK, D, TK, EXT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(L::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return -3;
     attr_set[dev] = true;
@@ -917,8 +1369,7 @@ static int launch_attention(const void* q, long long ldq, const void* k, const v
   }
   if (max_splits <= 1) a.sig = sig;
   dim3 grid((unsigned)num_work * (unsigned)Hkv);
-  (void)launch_pdl(attention_kernel<DK, D, TK, EXT, CAP>, grid, dim3(AttnShape<DK, TK>::kThreads), smem,
-                   stream, tq, tk, tv, a);
+  (void)launch_pdl(L::kernel(), grid, dim3(L::kThreads), smem, stream, tq, tk, tv, a);
   if (cudaGetLastError() != cudaSuccess) return -5;
   a.sig = sig;
   if (max_splits > 1) {
@@ -938,6 +1389,12 @@ extern "C" {
 
 #define AB200_ATTN_DISPATCH(EXT, CAP, ...)                                                 \
   do {                                                                                     \
+    if (tile_keys == kWideRows) {                                                          \
+      if (EXT) return -2;                                                                  \
+      if (D == 128) return launch_attention<128, 128, 128, false, false, true>(__VA_ARGS__); \
+      if (D == 64) return launch_attention<64, 64, 128, false, false, true>(__VA_ARGS__);  \
+      return -2;                                                                           \
+    }                                                                                      \
     const bool small = tile_keys == 64 && (block_size == 0 || block_size <= 64);           \
     if (D == 128) return small ? launch_attention<128, 128, 64, EXT, CAP>(__VA_ARGS__)     \
                                : launch_attention<128, 128, 128, EXT, CAP>(__VA_ARGS__);   \
@@ -951,7 +1408,8 @@ extern "C" {
 // [num_blocks(=rows), Hkv*D] with row stride ld_kv. `work` is an int32 [num_work, 8]
 // device array (layout above). With max_splits > 1, o_part/lse_part/tok_splits
 // must be given: o_part fp32 [max_splits, T, Hq, D], lse_part fp32 [max_splits, T, Hq].
-// tile_keys: 128 (prefill) or 64 (decode-shaped calls: few query rows per sequence).
+// tile_keys: 128 (prefill) or 64 (decode-shaped calls: few query rows per sequence); 256: 128-key tiles
+// and a work list whose items hold up to 256 / G tokens.
 int ab200_attention(const void* q, long long ldq, const void* k, const void* v, long long ld_kv,
                     long long num_blocks, int block_size, const void* block_tables, int max_blocks,
                     const void* work, int num_work, const void* tok_splits, int max_splits,

@@ -173,7 +173,7 @@ class BertEncoder:
         return ops.build_attention_metadata(list(seq_lens), list(seq_lens), None, 1,
                                             cfg.num_attention_heads, cfg.head_dim, self.device,
                                             causal=False, Hkv=cfg.num_attention_heads,
-                                            seq_rows=starts, allow_split=False)
+                                            seq_rows=starts, allow_split=False, wide=True)
 
     def embed(self, input_ids: torch.Tensor, positions: torch.Tensor, seq_lens: Sequence[int],
               starts: torch.Tensor, token_type_ids: Optional[torch.Tensor] = None,

@@ -387,7 +387,11 @@ class LayerListForCausalLM:
             rows = np.asarray(kv_lens) - np.asarray(lo)
             step.exp_plans[key] = ops.build_attention_metadata(
                 q_lens, kv_lens, None, 1, H, m.expand[1], self.device, Hkv=H,
-                seq_rows=np.cumsum(rows) - rows - np.asarray(lo), allow_split=False, mask=mask)
+                seq_rows=np.cumsum(rows) - rows - np.asarray(lo), allow_split=False, mask=mask,
+                # (the kernel with sinks and gates takes single tiles)
+                wide=m.expand[0] == m.expand[1] and not any(
+                    o.spec.sink is not None or o.spec.head_gate for o in self.mixers
+                    if isinstance(o, LatentMixer) and (o.spec.heads, o.expand, o.spec.mask) == key))
 
     def decode_plans(self, bucket: int, max_q: int, block_size: int) -> list:
         return [m.decode_plan(bucket, max_q, block_size)

@@ -822,15 +822,16 @@ class AttentionMetadata:
 
 def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: int = 148,
                         Hkv: int = 1, seq_rows=None, allow_split: bool = True,
-                        max_splits_cap: int = 16, mask=None, align: int = 1):
+                        max_splits_cap: int = 16, mask=None, align: int = 1, rows_per_item: int = 128):
     """Pure-host planner. Returns (work [n,8] int32 ndarray, tok_splits [T] int32, max_splits).
     ``mask`` (a MaskSpec): a tile's keys start at the first one its rows see, rounded down to a
     multiple of ``align`` (the cache's block size).
 
-    Query tokens of a sequence are cut into tiles of 128/G tokens. When the call has too few
+    Query tokens of a sequence are cut into tiles of 128/G tokens (``rows_per_item`` / G where the
+    kernel takes more rows per CTA). When the call has too few
     tiles to occupy the GPU (decode), the keys of each sequence are cut into up to 16 splits
     of whole 128-key tiles."""
-    tpt = 128 // G
+    tpt = rows_per_item // G
     if len(q_lens) >= 16 and max(q_lens) == 1 and min(q_lens) == 1:
         return _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split,
                                  max_splits_cap, mask, align)
@@ -947,14 +948,34 @@ def pick_tile_keys(q_lens, G: int) -> int:
     return 64 if q_lens and max(q_lens) * G <= 32 else 128
 
 
+WIDE_ROWS = 256   # rows of a work item of the kernel with two tiles of rows per CTA
+
+
+def wide_tiles_pay(q_lens, G: int, Hkv: int, D: int, num_sms: int = 148) -> bool:
+    """Whether a call should take 256 query rows per CTA. A CTA with two tiles takes 1.35 times as long as
+    one with a single tile and there are half as many of them, unless sequences are short: it pays
+    wherever the waves of CTAs become fewer (measured: 61 decodes beside 1987 tokens, 7 waves and 6, 159
+    and 140 us; four texts of 2048, 14 and 7, 291 and 186), and not in a single wave."""
+    tpt = 128 // G
+    if D not in (64, 128) or max(q_lens, default=0) <= tpt:
+        return False
+    one = sum(-(-q // tpt) for q in q_lens) * Hkv
+    two = sum(-(-q // (2 * tpt)) for q in q_lens) * Hkv
+    return -(-two // num_sms) < -(-one // num_sms)
+
+
 def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, causal=True,
                              Hkv=None, seq_rows=None, allow_split=True,
                              work_capacity: int | None = None, mask=None,
-                             align: int = 1) -> AttentionMetadata:
+                             align: int = 1, wide: bool = False) -> AttentionMetadata:
+    """``wide``: the calls that will use this plan take either arrangement of rows
+    (:func:`attention`, :func:`attention_contiguous`), so the better one may be chosen."""
     Hkv = Hkv if Hkv is not None else Hq // G
+    wide = wide and (mask is None or mask.kind == "causal") and wide_tiles_pay(q_lens, G, Hkv, D)
     work, tok_splits, max_splits = plan_attention_work(q_lens, kv_lens, G, causal, Hkv=Hkv,
                                                        seq_rows=seq_rows, allow_split=allow_split,
-                                                       mask=mask, align=align)
+                                                       mask=mask, align=align,
+                                                       rows_per_item=WIDE_ROWS if wide else 128)
     T = int(sum(q_lens))
     n = work.shape[0]
     if work_capacity is not None:
@@ -968,7 +989,7 @@ def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, ca
     meta.block_tables = block_tables
     meta.max_splits = max_splits
     meta.num_work = work.shape[0]
-    meta.tile_keys = pick_tile_keys(q_lens, G)
+    meta.tile_keys = WIDE_ROWS if wide else pick_tile_keys(q_lens, G)
     if max_splits > 1 and dev.type == "cuda":
         meta.o_part = torch.empty(max_splits, T, Hq, D, dtype=torch.float32, device=dev)
         meta.lse_part = torch.empty(max_splits, T, Hq, dtype=torch.float32, device=dev)
@@ -1072,6 +1093,7 @@ def attention_masked(q, k, v, meta: AttentionMetadata, Hq: int, Hkv: int, D: int
     same mask."""
     nat = _native()
     T = q.shape[0]
+    assert meta.tile_keys != WIDE_ROWS, "planned for another kernel"
     if out is None:
         out = torch.empty(T, Hq * D, dtype=q.dtype, device=q.device)
     bt = meta.block_tables if paged else None
@@ -1108,14 +1130,15 @@ def attention_contiguous(q, k, v, seq_lens, H: int, D: int, scale: float | None 
     if meta is None:
         starts = np.concatenate([[0], np.cumsum(seq_lens)[:-1]]).astype(np.int64)
         meta = build_attention_metadata(seq_lens, seq_lens, None, 1, H, D, q.device, causal=causal,
-                                        Hkv=H, seq_rows=starts, allow_split=False)
+                                        Hkv=H, seq_rows=starts, allow_split=False, wide=True)
     if out is None:
         out = torch.empty(T, H * D, dtype=q.dtype, device=q.device)
     assert k.stride(0) == v.stride(0)
     rc = nat.lib().ab200_attention(
         q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.shape[0], 0, None, 0,
         meta.work.data_ptr(), meta.num_work, None, 1, T, H, H, D, 1 if causal else 0, float(scale),
-        out.data_ptr(), out.stride(0), None, None, None, 128,
+        out.data_ptr(), out.stride(0), None, None, None,
+        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128,
         nat.status_buffer(q.device).data_ptr(), nat.stream_ptr())
     nat.check(rc, "attention_contiguous")
     launch_counter.add(1)

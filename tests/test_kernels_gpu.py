@@ -374,6 +374,30 @@ def test_paged_attention_split_kv():
     _close(out, exp, 2e-2, 2e-2)
 
 
+# two tiles of rows per CTA: a lone row in the second tile, a second tile that sees one key tile more
+# than the first, prefixes, keys that end at and beside a tile, split keys of which early rows see none,
+# padding rows, rows that are no multiple of a warp's
+@pytest.mark.parametrize("q_lens,kv_lens,Hq,Hkv,D,bs", [
+    ([33], [33], 8, 2, 128, 32), ([65, 40], [65, 168], 8, 2, 128, 64), ([300, 1, 64], [812, 640, 256], 8, 2, 128, 64),
+    ([257], [257], 4, 4, 64, 16), ([129, 255, 256], [129, 1255, 300], 2, 2, 64, 128), ([700], [700], 6, 2, 128, 32),
+])
+@pytest.mark.parametrize("split", [False, True])
+def test_paged_attention_wide(q_lens, kv_lens, Hq, Hkv, D, bs, split, monkeypatch):
+    q, kc, vc, bt = _paged_case(q_lens, kv_lens, Hq, Hkv, D, bs)
+    q = q * 4                      # maxima that keep moving
+    monkeypatch.setattr(ops, "wide_tiles_pay", lambda *a: True)
+    G = 1 << (Hq // Hkv - 1).bit_length()     # rows per token
+    meta = ops.build_attention_metadata(q_lens, kv_lens, bt, G, Hq, D, DEV, Hkv=Hkv, wide=True, allow_split=split)
+    assert meta.tile_keys == ops.WIDE_ROWS
+    lse = torch.empty(sum(q_lens), Hq, device=DEV, dtype=torch.float32)
+    out = ops.attention(q, kc, vc, meta, Hq, Hkv, D, lse_out=lse)
+    ops.check_status()
+    exp, lse_ref = ref.attention(q, kc, vc, bt, q_lens, kv_lens, Hq, Hkv, D, 1 / math.sqrt(D),
+                                 return_lse=True)
+    _close(out, exp, 2e-2, 2e-2)
+    _close(lse, lse_ref, 2e-2, 1e-2)
+
+
 @pytest.mark.parametrize("H,D,seq_lens", [(12, 64, [50, 128, 3, 512]), (4, 128, [77, 300])])
 def test_encoder_attention(H, D, seq_lens):
     T = sum(seq_lens)

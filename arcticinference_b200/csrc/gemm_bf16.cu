@@ -1198,6 +1198,20 @@ static int pick_tile_width(int tiles_a, int N, int kblocks, int units, bool pair
   return best;
 }
 
+// The plan of a size, made once (a hundred candidates cost the host 2 us, as much as the launch).
+static FewPlan few_plan_of(int M, int N, int kblocks, int group_max, int sms) {
+  static std::mutex mu;
+  static std::unordered_map<uint64_t, FewPlan> plans;
+  const uint64_t key = ((uint64_t)M << 54) ^ ((uint64_t)group_max << 50) ^ ((uint64_t)N << 20) ^ (uint64_t)kblocks;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = plans.find(key);
+  if (it != plans.end()) return it->second;
+  const FewPlan plan = plan_few(M, N, kblocks, group_max, sms, cluster_capacity);
+  if (plans.size() > 8192) plans.clear();
+  plans.emplace(key, plan);
+  return plan;
+}
+
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 32;
   while (p < v) p <<= 1;
@@ -1290,7 +1304,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
       (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
     const int elems = fp8 ? kBlockKFp8 : kBlockK;
     const int kblocks = (K + elems - 1) / elems;
-    const FewPlan plan = plan_few(M, N, kblocks, K % elems == 0 ? 4 : 1, num_sms(), cluster_capacity);
+    const FewPlan plan = few_plan_of(M, N, kblocks, K % elems == 0 ? 4 : 1, num_sms());
     if (plan.bn > 0) {
       FewArgs f;
       f.scale_x = scale_x;

@@ -79,6 +79,9 @@ int ab200_bert_embed_ln(const void* ids, const void* positions, const void* type
                         const void* beta, void* out, long long T, int hidden, long long vocab,
                         long long max_pos, long long n_types, float eps, int* status,
                         cudaStream_t stream);
+int ab200_attention_short(const void* q, long long ldq, const void* k, const void* v, long long ld_kv,
+                          const void* work, int num_work, int heads, int max_len, float scale, void* out,
+                          long long ldo, cudaStream_t stream);
 int ab200_pool_normalize(const void* h, long long ld, const void* starts, void* out, int n_seqs,
                          int hidden, int mode, int normalize, cudaStream_t stream);
 // kv_cache.cu

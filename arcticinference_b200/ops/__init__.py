@@ -948,6 +948,7 @@ def pick_tile_keys(q_lens, G: int) -> int:
     return 64 if q_lens and max(q_lens) * G <= 32 else 128
 
 
+SHORT_TOKENS = 128   # longest sequence of the kernel for many short ones
 WIDE_ROWS = 256   # rows of a work item of the kernel with two tiles of rows per CTA
 
 
@@ -1134,6 +1135,14 @@ def attention_contiguous(q, k, v, seq_lens, H: int, D: int, scale: float | None 
     if out is None:
         out = torch.empty(T, H * D, dtype=q.dtype, device=q.device)
     assert k.stride(0) == v.stride(0)
+    longest = max(max(meta.q_lens), max(meta.kv_lens))
+    if not causal and D == 64 and longest <= SHORT_TOKENS:
+        rc = nat.lib().ab200_attention_short(
+            q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), meta.work.data_ptr(),
+            meta.num_work, H, longest, float(scale), out.data_ptr(), out.stride(0), nat.stream_ptr())
+        nat.check(rc, "attention_short")
+        launch_counter.add(1)
+        return out
     rc = nat.lib().ab200_attention(
         q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.shape[0], 0, None, 0,
         meta.work.data_ptr(), meta.num_work, None, 1, T, H, H, D, 1 if causal else 0, float(scale),

@@ -398,6 +398,23 @@ def test_paged_attention_wide(q_lens, kv_lens, Hq, Hkv, D, bs, split, monkeypatc
     _close(lse, lse_ref, 2e-2, 1e-2)
 
 
+# sequences of at most 128 tokens: every register size, ends of 16-row and 16-key groups
+@pytest.mark.parametrize("seq_lens", [[1], [32, 1, 31], [33, 17, 64, 50], [65, 96, 2], [97, 128, 127, 112]])
+def test_encoder_attention_short(seq_lens):
+    H, D, T = 3, 64, sum(seq_lens)
+    qkv = _rand(T, 3 * H * D)
+    out = ops.attention_contiguous(qkv[:, :H * D], qkv[:, H * D:2 * H * D], qkv[:, 2 * H * D:], seq_lens, H, D)
+    at = 0
+    for n in seq_lens:
+        q, k, v = (x.double() for x in qkv[at:at + n].view(n, 3, H, D).permute(1, 2, 0, 3))
+        w = torch.softmax(q @ k.mT / math.sqrt(D), -1)
+        # probabilities and the result are rounded to bf16 (2^-8 of the value each)
+        bound = 2.0 ** -8 * ((w @ v).abs() + w @ v.abs()) + 1e-5
+        got = out[at:at + n].double().view(n, H, D).transpose(0, 1)
+        assert ((got - w @ v).abs() <= bound).all(), n
+        at += n
+
+
 @pytest.mark.parametrize("H,D,seq_lens", [(12, 64, [50, 128, 3, 512]), (4, 128, [77, 300])])
 def test_encoder_attention(H, D, seq_lens):
     T = sum(seq_lens)

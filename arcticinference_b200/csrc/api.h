@@ -82,6 +82,12 @@ int ab200_bert_embed_ln(const void* ids, const void* positions, const void* type
 int ab200_attention_short(const void* q, long long ldq, const void* k, const void* v, long long ld_kv,
                           const void* work, int num_work, int heads, int max_len, float scale, void* out,
                           long long ldo, cudaStream_t stream);
+typedef struct Ab200BertLayer {
+  const void *wqkv, *bqkv, *wo, *bo, *ln1_g, *ln1_b, *wi, *bi, *wd, *bd, *ln2_g, *ln2_b;
+} Ab200BertLayer;
+int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void* x, void* wide, void* a,
+                      int T, int hidden, int inter, int heads, int D, float eps, const void* work,
+                      int num_work, int tile_keys, int max_len, int* status, cudaStream_t stream);
 int ab200_pool_normalize(const void* h, long long ld, const void* starts, void* out, int n_seqs,
                          int hidden, int mode, int normalize, cudaStream_t stream);
 // kv_cache.cu

@@ -361,6 +361,46 @@ int ab200_attention_short(const void* q, long long ldq, const void* k, const voi
              : -5;
 }
 
+// All layers of an encoder over a packed batch: h [T, hidden] in and out; x [T, hidden], a [T, hidden]
+// and wide [T, max(3 hidden, inter)] are scratch. One call enqueues the seven kernels of every layer:
+// from Python each launch costs 17 us of the host, more than the kernel takes for a short text.
+int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void* x, void* wide, void* a,
+                      int T, int hidden, int inter, int heads, int D, float eps, const void* work,
+                      int num_work, int tile_keys, int max_len, int* status, cudaStream_t stream) {
+  if (T <= 0 || n_layers <= 0) return 0;
+  if (layers == nullptr || heads * D != hidden) return -2;
+  const float scale = 1.f / sqrtf((float)D);
+  char* qkv = reinterpret_cast<char*>(wide);
+  const size_t part = (size_t)hidden * 2;   // bytes
+  for (int l = 0; l < n_layers; ++l) {
+    const Ab200BertLayer& w = layers[l];
+    int rc = ab200_linear_bf16(h, hidden, w.wqkv, hidden, wide, 3 * hidden, T, 3 * hidden, hidden, w.bqkv,
+                               nullptr, 0, 0, nullptr, 0, 0, status, stream);
+    if (rc != 0) return rc;
+    rc = D == kShortDim && max_len <= kShortLen
+             ? ab200_attention_short(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, work, num_work,
+                                     heads, max_len, scale, a, hidden, stream)
+             : ab200_attention(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, T, 0, nullptr, 0, work,
+                               num_work, nullptr, 1, T, heads, heads, D, 0, scale, a, hidden, nullptr, nullptr,
+                               nullptr, tile_keys, status, stream);
+    if (rc != 0) return rc;
+    rc = ab200_linear_bf16(a, hidden, w.wo, hidden, x, hidden, T, hidden, hidden, w.bo, h, hidden, 0,
+                           nullptr, 0, 0, status, stream);
+    if (rc != 0) return rc;
+    rc = ab200_layernorm(x, nullptr, w.ln1_g, w.ln1_b, h, T, hidden, eps, stream);
+    if (rc != 0) return rc;
+    rc = ab200_linear_bf16(h, hidden, w.wi, hidden, wide, inter, T, inter, hidden, w.bi, nullptr, 0, 1,
+                           nullptr, 0, 0, status, stream);
+    if (rc != 0) return rc;
+    rc = ab200_linear_bf16(wide, inter, w.wd, inter, x, hidden, T, hidden, inter, w.bd, h, hidden, 0,
+                           nullptr, 0, 0, status, stream);
+    if (rc != 0) return rc;
+    rc = ab200_layernorm(x, nullptr, w.ln2_g, w.ln2_b, h, T, hidden, eps, stream);
+    if (rc != 0) return rc;
+  }
+  return 0;
+}
+
 int ab200_pool_normalize(const void* h, long long ld, const void* starts, void* out, int n_seqs,
                          int hidden, int mode, int normalize, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;

@@ -38,6 +38,10 @@ class BertLayerWeights:
         for s in self.__slots__:
             setattr(self, s, None)
 
+    def in_order(self) -> tuple:
+        """The weights in the order of the native call's ``Ab200BertLayer``."""
+        return tuple(getattr(self, s) for s in self.__slots__)
+
 
 def random_bert_state(cfg: ModelConfig, seed: int, std: float, device, dtype) -> Iterator:
     """(name, tensor) pairs of a random checkpoint in Hugging Face naming."""
@@ -156,6 +160,9 @@ class BertEncoder:
                               self.emb_g, self.emb_b, eps)
         if attn_meta is None and h.is_cuda:
             attn_meta = self.attention_metadata(seq_lens)
+        if h.is_cuda and h.dtype == torch.bfloat16:
+            return ops.bert_layers(h, [lw.in_order() for lw in self.layers], cfg.intermediate_size, Hh, D,
+                                   eps, attn_meta)
         for lw in self.layers:
             qkv = ops.linear(h, lw.wqkv, bias=lw.bqkv)
             a = ops.attention_contiguous(qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:], seq_lens, Hh, D,

@@ -8,6 +8,7 @@ also the oracles of the numerics tests.
 
 from __future__ import annotations
 
+import ctypes
 import math
 import sys
 from dataclasses import dataclass, field
@@ -1117,6 +1118,30 @@ def attention_masked(q, k, v, meta: AttentionMetadata, Hq: int, Hkv: int, D: int
     nat.check(rc, "attention_masked")
     launch_counter.add(2 if meta.max_splits > 1 else 1)
     return out
+
+
+def bert_layers(h: torch.Tensor, layers, inter: int, heads: int, D: int, eps: float,
+                meta: AttentionMetadata) -> torch.Tensor:
+    """Encoder layers over a packed batch, ``h`` [T, heads * D] (overwritten) in and out, all of them
+    enqueued by one native call. ``layers``: a tuple per layer of the weights in the order of
+    ``Ab200BertLayer``, contiguous and of h's type (bf16)."""
+    nat = _native()
+    T, H = h.shape
+    shapes = ((3 * H, H), (3 * H,), (H, H), (H,), (H,), (H,), (inter, H), (inter,), (H, inter), (H,), (H,), (H,))
+    for lw in layers:
+        for t, shape in zip(lw, shapes, strict=True):
+            assert t.shape == shape and t.dtype == h.dtype == torch.bfloat16 and t.is_contiguous()
+    ptrs = (ctypes.c_void_p * (len(layers) * len(shapes)))(*[t.data_ptr() for lw in layers for t in lw])
+    x, a = torch.empty_like(h), torch.empty_like(h)
+    wide = torch.empty(T, max(3 * H, inter), dtype=h.dtype, device=h.device)
+    rc = nat.lib().ab200_bert_layers(
+        ptrs, len(layers), h.data_ptr(), x.data_ptr(), wide.data_ptr(), a.data_ptr(), T, H, inter, heads,
+        D, float(eps), meta.work.data_ptr(), meta.num_work,
+        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128, max(max(meta.q_lens), max(meta.kv_lens)),
+        nat.status_buffer(h.device).data_ptr(), nat.stream_ptr())
+    nat.check(rc, "bert_layers T=%d" % T)
+    launch_counter.add(7 * len(layers))
+    return h
 
 
 def attention_contiguous(q, k, v, seq_lens, H: int, D: int, scale: float | None = None,

@@ -415,6 +415,28 @@ def test_encoder_attention_short(seq_lens):
         at += n
 
 
+@pytest.mark.parametrize("seq_lens", [[1], [50, 7], [128, 129], [300, 512]])
+def test_bert_layers_native(seq_lens):
+    """The layers that one native call enqueues are those of the ops, kernel by kernel."""
+    H, I, D, n, T = 192, 320, 64, 2, sum(seq_lens)
+    w = lambda *s: _rand(*s, scale=1.0 / math.sqrt(s[-1]))    # noqa: E731
+    layers = [(w(3 * H, H), _rand(3 * H), w(H, H), _rand(H), _rand(H), _rand(H), w(I, H), _rand(I), w(H, I), _rand(H),
+               _rand(H), _rand(H)) for _ in range(n)]
+    h = _rand(T, H)
+    starts = [sum(seq_lens[:i]) for i in range(len(seq_lens))]
+    meta = ops.build_attention_metadata(seq_lens, seq_lens, None, 1, H // D, D, DEV, causal=False, Hkv=H // D,
+                                        seq_rows=starts, allow_split=False, wide=True)
+    y = h
+    for wqkv, bqkv, wo, bo, g1, b1, wi, bi, wd, bd, g2, b2 in layers:
+        qkv = ops.linear(y, wqkv, bias=bqkv)
+        a = ops.attention_contiguous(qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:], seq_lens, H // D, D, meta=meta)
+        y = ops.layernorm(ops.linear(a, wo, bias=bo, residual=y), g1, b1, 1e-12)
+        u = ops.linear(y, wi, bias=bi, act="gelu")
+        y = ops.layernorm(ops.linear(u, wd, bias=bd, residual=y), g2, b2, 1e-12)
+    assert torch.equal(ops.bert_layers(h.clone(), layers, I, H // D, D, 1e-12, meta), y)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("H,D,seq_lens", [(12, 64, [50, 128, 3, 512]), (4, 128, [77, 300])])
 def test_encoder_attention(H, D, seq_lens):
     T = sum(seq_lens)

@@ -55,6 +55,8 @@ int ab200_linear_bf16(const void* x, long long ldx, const void* w, long long ldw
                       long long ldo, int M, int N, int K, const void* bias, const void* residual,
                       long long ldr, int act, void* workspace, size_t workspace_bytes,
                       int force_splits, int* status, cudaStream_t stream);
+int ab200_linear_silu(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, int M,
+                      int inter, int K, int* status, cudaStream_t stream);
 int ab200_gemm_bf16_nn(const void* x, long long ldx, const void* wt, long long ldw, void* out,
                        long long ldo, int M, int N, int K, int* status, cudaStream_t stream);
 

@@ -388,9 +388,12 @@ class LlamaForCausalLM(LlamaModel):
         return self._linear_reduce(attn, self._o_w(lw, mode), mode, wait)
 
     def _mlp_block(self, lw, x, mode):
-        gu = ops.linear(x, self._gu_w(lw, mode))
+        w = self._gu_w(lw, mode)
         nblk = self.n_stored if (mode == "sp" or self.n_stored == 1) else 1
-        act = ops.silu_mul_blocked(gu, nblk, quant=self.act_quant)
+        if nblk == 1 and not self.act_quant and isinstance(w, torch.Tensor) and isinstance(x, torch.Tensor):
+            act = ops.linear_silu(x, w)
+        else:
+            act = ops.silu_mul_blocked(ops.linear(x, w), nblk, quant=self.act_quant)
         return self._linear_reduce(act, self._down_w(lw, mode), mode)
 
     def _linear_reduce(self, x, w, mode, wait=None):

@@ -407,6 +407,27 @@ def linear(x: torch.Tensor, w, bias=None, residual=None, act=None, out=None,
     return out
 
 
+def linear_silu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """silu(x @ w[:I].T) * (x @ w[I:].T) for w [2 I, K] (gate rows, then up rows): one kernel for more than
+    256 bf16 tokens, :func:`linear` and :func:`silu_mul` otherwise. (With few tokens the weights bound the
+    product and the activation's pass is short.)"""
+    inter = w.shape[0] // 2
+    if isinstance(x, torch.Tensor) and x.is_cuda and x.shape[0] > 256 and \
+            x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == w.stride(1) == 1 and \
+            x.shape[1] % 8 == 0 and inter % 8 == 0 and inter >= 128:
+        nat = _native()
+        M, K = x.shape
+        out = torch.empty(M, inter, dtype=x.dtype, device=x.device)
+        rc = nat.lib().ab200_linear_silu(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
+                                         out.stride(0), M, inter, K, nat.status_buffer(x.device).data_ptr(),
+                                         nat.stream_ptr())
+        if rc != -6:
+            nat.check(rc, "linear_silu M=%d I=%d K=%d" % (M, inter, K))
+            launch_counter.add(1)
+            return out
+    return silu_mul(linear(x, w))
+
+
 def _linear_exact(x: torch.Tensor, w: torch.Tensor, out=None) -> torch.Tensor:
     nat = _native()
     assert x.dtype == w.dtype and x.dtype in (torch.bfloat16, torch.float32)

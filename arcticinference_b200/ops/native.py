@@ -95,6 +95,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "ab200_rmsnorm": (I, [P, LL, P, P, P, LL, LL, I, F, P]),
         "ab200_attention_short": (I, [P, LL, P, P, LL, P, I, I, I, F, P, LL, P]),
         "ab200_bert_layers": (I, [P, I, P, P, P, P, I, I, I, I, I, F, P, I, I, I, P, P]),
+        "ab200_linear_silu": (I, [P, LL, P, LL, P, LL, I, I, I, P, P]),
         "ab200_layernorm": (I, [P, P, P, P, P, LL, I, F, P]),
         "ab200_silu_mul": (I, [P, P, LL, I, I, P]),
         "ab200_rope_cache": (I, [P, LL, P, P, P, P, P, LL, I, I, I, I, LL, I, P, P]),

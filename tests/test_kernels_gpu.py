@@ -258,6 +258,20 @@ def test_linear_few_tokens(M, N, K, fp8):
     _check_linear(M, N, K, fp8)
 
 
+# gate / up rows of one tile in the two CTAs of a pair: ends of the tiles, more tiles than pairs
+@pytest.mark.parametrize("M,inter,K", [(257, 128, 64), (300, 136, 80), (513, 1416, 768), (5000, 2040, 256)])
+def test_linear_silu(M, inter, K):
+    x, w = _rand(M, K), _rand(2 * inter, K, scale=1.0 / math.sqrt(K))
+    before = ops.count_launches()
+    out = ops.linear_silu(x, w)
+    assert ops.count_launches() == before + 1
+    ops.check_status()
+    z = x.double() @ w.double().t()
+    y = torch.nn.functional.silu(z[:, :inter]) * z[:, inter:]
+    # one rounding to bf16; fp32 sums and the fast exponential before it
+    assert ((out.double() - y).abs() <= y.abs() * 2.0 ** -8 + 2e-4).all()
+
+
 # CTA pairs: ends of 256-row tiles, of each tile width and of the ring of stages, one tile, several
 # groups of rows of tiles, more tiles than pairs
 @pytest.mark.parametrize("fp8", [False, True])

@@ -1189,7 +1189,7 @@ __global__ void attention_merge_kernel(const float* __restrict__ o_part,
   const long long tok = blockIdx.x;
   const int ns = tok_splits[tok];
   if (ns <= 1) {
-    tail_signal(pa.sig, gridDim.x);
+    tail_signal(pa.sig, gridDim.x * gridDim.y);
     return;
   }
   long long out_row = tok;
@@ -1197,28 +1197,43 @@ __global__ void attention_merge_kernel(const float* __restrict__ o_part,
     out = pa.peer_out[tok / pa.peer_tokens];
     out_row = tok % pa.peer_tokens;
   }
-  for (int idx = threadIdx.x; idx < Hq * (D / 4); idx += blockDim.x) {
+  // One output vector per thread, the heads over the blocks' second index (a lone token's merge was a
+  // chain of 8 vectors x 16 splits in one block, 9.6 us), four splits' loads in flight at a time.
+  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < Hq * (D / 4); idx += gridDim.y * blockDim.x) {
     const int head = idx / (D / 4);
     const int d4 = (idx % (D / 4)) * 4;
-    float mx = -INFINITY;
-    for (int s = 0; s < ns; ++s) mx = fmaxf(mx, lse_part[((long long)s * T + tok) * Hq + head]);
     float sink = -INFINITY;
-    if (EXT && pa.sink != nullptr) {
-      sink = pa.sink[head];
-      mx = fmaxf(mx, sink);
-    }
+    if (EXT && pa.sink != nullptr) sink = pa.sink[head];
+    float mx = sink;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float wsum = (EXT && sink != -INFINITY) ? __expf(sink - mx) : 0.f;
-    for (int s = 0; s < ns; ++s) {
-      const float lse = lse_part[((long long)s * T + tok) * Hq + head];
-      const float w = (lse == -INFINITY) ? 0.f : __expf(lse - mx);
-      const float4 v =
-          *reinterpret_cast<const float4*>(o_part + (((long long)s * T + tok) * Hq + head) * D + d4);
-      acc.x += w * v.x;
-      acc.y += w * v.y;
-      acc.z += w * v.z;
-      acc.w += w * v.w;
-      wsum += w;
+    float wsum = sink != -INFINITY ? 1.f : 0.f;
+    const long long row = tok * Hq + head, step = T * Hq;   // rows of o_part and lse_part
+    for (int s0 = 0; s0 < ns; s0 += 4) {
+      float lse[4];
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        lse[i] = -INFINITY;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0 + i < ns) {
+          lse[i] = lse_part[(s0 + i) * step + row];
+          v[i] = *reinterpret_cast<const float4*>(o_part + ((s0 + i) * step + row) * D + d4);
+        }
+      }
+      const float top = fmaxf(fmaxf(fmaxf(lse[0], lse[1]), fmaxf(lse[2], lse[3])), mx);
+      const float keep = mx == -INFINITY ? 0.f : __expf(mx - top);
+      acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+      wsum *= keep;
+      mx = top;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float w = (lse[i] == -INFINITY) ? 0.f : __expf(lse[i] - mx);
+        acc.x += w * v[i].x;
+        acc.y += w * v[i].y;
+        acc.z += w * v[i].z;
+        acc.w += w * v[i].w;
+        wsum += w;
+      }
     }
     const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
     if (EXT && pa.gate != nullptr) {
@@ -1240,7 +1255,13 @@ __global__ void attention_merge_kernel(const float* __restrict__ o_part,
     *reinterpret_cast<uint2*>(out + out_row * ldo + (long long)head * D + d4) = q;
     if (lse_out && d4 == 0) lse_out[tok * Hq + head] = wsum > 0.f ? mx + logf(wsum) : -INFINITY;
   }
-  tail_signal(pa.sig, gridDim.x);
+  tail_signal(pa.sig, gridDim.x * gridDim.y);
+}
+
+// A block per token and part of its heads; with many tokens, of which most are in one piece, fewer parts.
+static dim3 merge_grid(long long T, int Hq, int D) {
+  const long long parts = (Hq * (D / 4) + 127) / 128, fit = 148 * 8 / T;
+  return dim3((unsigned)T, (unsigned)(fit < 1 ? 1 : fit < parts ? fit : parts));
 }
 
 struct AttnExt {
@@ -1373,7 +1394,7 @@ static int launch_attention(const void* q, long long ldq, const void* k, const v
   if (cudaGetLastError() != cudaSuccess) return -5;
   a.sig = sig;
   if (max_splits > 1) {
-    (void)launch_pdl(attention_merge_kernel<D, EXT>, dim3((unsigned)T), dim3(128), 0, stream, o_part,
+    (void)launch_pdl(attention_merge_kernel<D, EXT>, merge_grid(T, Hq, D), dim3(128), 0, stream, o_part,
                      lse_part, tok_splits, T, Hq, reinterpret_cast<__nv_bfloat16*>(out), ldo,
                      lse_out, a);
     if (cudaGetLastError() != cudaSuccess) return -5;
@@ -1492,7 +1513,7 @@ int ab200_attention_merge(const void* o_part, const void* lse_part, const void* 
            : D == 384 ? (ext ? attention_merge_kernel<384, true> : attention_merge_kernel<384, false>)
                       : (ext ? attention_merge_kernel<512, true> : attention_merge_kernel<512, false>);
   if (D != 128 && D != 256 && D != 384 && D != 512) return -2;
-  return launch_pdl(k, dim3((unsigned)T), dim3(D >= 256 ? 256 : 128), 0, stream,
+  return launch_pdl(k, merge_grid(T, Hq, D), dim3(128), 0, stream,
                     reinterpret_cast<const float*>(o_part), reinterpret_cast<const float*>(lse_part),
                     reinterpret_cast<const int*>(tok_splits), T, Hq,
                     reinterpret_cast<__nv_bfloat16*>(out), ldo, (float*)nullptr, a) == cudaSuccess

@@ -842,9 +842,23 @@ class AttentionMetadata:
                    if t is not None)
 
 
+def decode_splits(ctas: int, key_tiles: int, slots: int, most: int = 16) -> int:
+    """Pieces that each of ``ctas`` equal CTAs of a decode call (two per SM, 64-key stages) should be cut
+    into. A CTA streams a 128-key tile in 3 us however few run beside it (all slots together then
+    stream at the copy bandwidth) and costs 4 us besides; pieces cost a merge. 192 CTAs of 24 tiles on 296
+    slots: 67 us whole, 62 in three. At most two waves of pieces."""
+    best, best_us = 1, 0.0
+    for ns in range(1, max(1, min(most, key_tiles // 2, 2 * slots // max(1, ctas))) + 1):
+        us = -(-ctas * ns // slots) * (-(-key_tiles // ns) * 3.0 + 4.0) + (3.0 if ns > 1 else 0.0)
+        if ns == 1 or us < best_us - 1.0:
+            best, best_us = ns, us
+    return best
+
+
 def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: int = 148,
                         Hkv: int = 1, seq_rows=None, allow_split: bool = True,
-                        max_splits_cap: int = 16, mask=None, align: int = 1, rows_per_item: int = 128):
+                        max_splits_cap: int = 16, mask=None, align: int = 1, rows_per_item: int = 128,
+                        fill_slots: bool = False):
     """Pure-host planner. Returns (work [n,8] int32 ndarray, tok_splits [T] int32, max_splits).
     ``mask`` (a MaskSpec): a tile's keys start at the first one its rows see, rounded down to a
     multiple of ``align`` (the cache's block size).
@@ -852,18 +866,20 @@ def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: i
     Query tokens of a sequence are cut into tiles of 128/G tokens (``rows_per_item`` / G where the
     kernel takes more rows per CTA). When the call has too few
     tiles to occupy the GPU (decode), the keys of each sequence are cut into up to 16 splits
-    of whole 128-key tiles."""
+    of whole 128-key tiles; with ``fill_slots`` (calls of the 64-key
+    kernel, whatever padding they carry) the number follows from how CTAs of the decode
+    kernel share the SMs (:func:`decode_splits`)."""
     tpt = rows_per_item // G
     if len(q_lens) >= 16 and max(q_lens) == 1 and min(q_lens) == 1:
         return _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split,
-                                 max_splits_cap, mask, align)
+                                 max_splits_cap, mask, align, fill_slots)
     first = (lambda pos: 0) if mask is None else \
         (lambda pos: int(mask.first_key(pos)) // align * align)
     rows = []
     T = int(sum(q_lens))
     tok_splits = np.ones(max(T, 1), dtype=np.int32)
     n_tiles_total = sum((ql + tpt - 1) // tpt for ql in q_lens)
-    if q_lens and max(q_lens) * G <= 32:
+    if fill_slots or q_lens and max(q_lens) * G <= 32:
         num_sms *= 2  # decode-shaped calls run two CTAs per SM (64-key tiles)
     t0 = 0
     max_splits = 1
@@ -876,6 +892,8 @@ def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: i
         ns = 1
         if allow_split and n_tiles_total * Hkv < num_sms and key_tiles > 4:
             want = max(1, num_sms // max(1, n_tiles_total * Hkv))
+            if fill_slots:
+                want = decode_splits(n_tiles_total * Hkv, key_tiles, num_sms, int(min(16, max_splits_cap)))
             ns = int(min(16, max_splits_cap, want, max(1, key_tiles // 2)))
         tiles_per_split = (key_tiles + ns - 1) // ns
         ns = (key_tiles + tiles_per_split - 1) // tiles_per_split
@@ -916,7 +934,7 @@ def tail_split_plan(n_seqs: int, Hkv: int, slots: int, max_splits: int = 4):
 
 
 def _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split, max_splits_cap,
-                      mask=None, align=1):
+                      mask=None, align=1, fill_slots=False):
     """The planner above for the one-token-per-sequence case, on arrays (same rows, same
     order): a serving step with a thousand sequences must not spend milliseconds here."""
     kl = np.asarray(kv_lens, dtype=np.int64)
@@ -928,6 +946,8 @@ def _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split, m
     ns = np.ones(R, dtype=np.int64)
     if allow_split and R * Hkv < num_sms:
         want = max(1, num_sms // max(1, R * Hkv))
+        if G <= 32 and fill_slots:
+            want = decode_splits(R * Hkv, int(key_tiles.mean()), num_sms, int(min(16, max_splits_cap)))
         cand = np.minimum(np.minimum(16, max_splits_cap), np.minimum(want, np.maximum(1, key_tiles // 2)))
         ns = np.where(key_tiles > 4, cand, 1)
     elif allow_split and max_splits_cap > 1:
@@ -998,7 +1018,8 @@ def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, ca
     work, tok_splits, max_splits = plan_attention_work(q_lens, kv_lens, G, causal, Hkv=Hkv,
                                                        seq_rows=seq_rows, allow_split=allow_split,
                                                        mask=mask, align=align,
-                                                       rows_per_item=WIDE_ROWS if wide else 128)
+                                                       rows_per_item=WIDE_ROWS if wide else 128,
+                                                       fill_slots=not wide and pick_tile_keys(q_lens, G) == 64)
     T = int(sum(q_lens))
     n = work.shape[0]
     if work_capacity is not None:
@@ -1030,14 +1051,24 @@ class DecodePlan:
         # enough KV splits to occupy the GPU when the batch is small; for a large batch the
         # sequences of the last, partly filled wave of CTAs are cut (tail_split_plan)
         small_tiles = max_q * G <= 32 and block_size <= 64
+        slots = 148 * (2 if small_tiles else 1)
         self.splits = int(max(1, min(16, 148 // max(1, bucket * Hkv))))
-        self.work_cap = bucket * self.splits + 1
-        n_cut, pieces = tail_split_plan(bucket, Hkv, 148 * (2 if small_tiles else 1))
+        n_cut, pieces = tail_split_plan(bucket, Hkv, slots)
         if self.splits == 1 and n_cut > 0 and max_q == 1:
             self.splits = pieces
-            self.work_cap = bucket + n_cut * (pieces - 1) + 1
+        if small_tiles and bucket > 1 and -(-bucket // 4) * Hkv < slots:
+            # drafts to verify: as many tokens from a quarter of the sequences, which are cut again
+            self.splits = max(self.splits, 4)
+        # pieces that any number of sequences of this bucket can come to
+        self.work_cap = 1 + max(self._pieces(n, Hkv, slots, small_tiles) for n in range(1, bucket + 1))
         self.tile_keys = 64 if small_tiles else 128
         self.meta = AttentionMetadata([], [], bucket)
+
+    def _pieces(self, n: int, Hkv: int, slots: int, small: bool) -> int:
+        if n * Hkv < slots:
+            return min(n * self.splits, max(n, 2 * slots // Hkv)) if small else n * self.splits
+        n_cut, pieces = tail_split_plan(n, Hkv, slots, min(4, self.splits))
+        return n + n_cut * (pieces - 1)
 
     @property
     def int32_words(self) -> int:
@@ -1046,7 +1077,7 @@ class DecodePlan:
     def plan(self, q_lens, kv_lens):
         return plan_attention_work(q_lens, kv_lens, self.G, True, Hkv=self.Hkv,
                                    max_splits_cap=self.splits, mask=self.mask,
-                                   align=self.block_size)
+                                   align=self.block_size, fill_slots=self.tile_keys == 64)
 
     def bind(self, host, dev: torch.Tensor, block_tables: torch.Tensor) -> None:
         """``host`` (numpy) and ``dev``: this plan's ``int32_words`` of the staging buffers."""

@@ -50,3 +50,28 @@ def test_small_decode_batch_is_split_to_occupy_the_gpu():
     assert max_splits > 1
     _covered(work, 16, kv)
     assert np.all(work[:, 2] == 1)
+
+
+def test_decode_splits_fill_at_most_two_waves():
+    for ctas in (1, 8, 24, 64, 150, 192, 295):
+        for tiles in (1, 4, 9, 24, 300):
+            ns = ops.decode_splits(ctas, tiles, 296)
+            assert 1 <= ns <= 16 and (ns == 1 or ctas * ns <= 592 and ns <= tiles // 2)
+    assert ops.decode_splits(192, 24, 296) == 3
+
+
+def test_captured_decode_plan_holds_every_mix_of_requests():
+    rng = np.random.default_rng(0)
+    for bucket in (1, 2, 8, 17, 32, 96, 128, 160):
+        for hkv in (1, 8):
+            plan = ops.DecodePlan(4, 4 * hkv, hkv, 128, bucket, 1, 64)
+            for _ in range(40):
+                n = int(rng.integers(1, bucket + 1))
+                q = [1] * n if rng.random() < 0.5 else [4] * max(1, n // 4)
+                q = q if sum(q) <= bucket else [1]
+                kv = [int(k) for k in rng.integers(5, 9000, len(q))]
+                if sum(q) < bucket:        # the padding tokens' own sequence
+                    q, kv = q + [bucket - sum(q)], kv + [bucket - sum(q)]
+                work, splits, most = plan.plan(q, kv)
+                assert work.shape[0] <= plan.work_cap and most <= plan.splits
+                _covered(work, len(q), kv) if max(q) == 1 else None

@@ -451,6 +451,23 @@ def test_bert_layers_native(seq_lens):
     ops.check_status()
 
 
+@pytest.mark.parametrize("T,ns", [(1, 16), (3, 1), (5, 5), (700, 3)])
+def test_attention_merge_pieces(T, ns):
+    Hq, Hkv, D, n = 6, 2, 128, 140
+    q_lens, kv_lens = [1] * T, [n + 128 * 2 * ns - 1] * T
+    q, kc, vc, bt = _paged_case(q_lens, kv_lens, Hq, Hkv, D, 64)
+    meta = ops.build_attention_metadata(q_lens, kv_lens, bt, 4, Hq, D, DEV, Hkv=Hkv)
+    rows = [(t, t, 1, kv_lens[t] - 1, s * 256, min(kv_lens[t], (s + 1) * 256) if s < ns - 1 else kv_lens[t], s, ns)
+            for t in range(T) for s in range(ns)]
+    meta.work, meta.num_work = torch.tensor(rows, dtype=torch.int32, device=DEV), len(rows)
+    meta.tok_splits, meta.max_splits = torch.full((T,), ns, dtype=torch.int32, device=DEV), ns
+    meta.o_part = torch.empty(ns, T, Hq, D, device=DEV)
+    meta.lse_part = torch.empty(ns, T, Hq, device=DEV)
+    out = ops.attention(q, kc, vc, meta, Hq, Hkv, D)
+    ops.check_status()
+    _close(out, ref.attention(q, kc, vc, bt, q_lens, kv_lens, Hq, Hkv, D, 1 / math.sqrt(D)), 2e-2, 2e-2)
+
+
 @pytest.mark.parametrize("H,D,seq_lens", [(12, 64, [50, 128, 3, 512]), (4, 128, [77, 300])])
 def test_encoder_attention(H, D, seq_lens):
     T = sum(seq_lens)

@@ -340,9 +340,10 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* 
       ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-// Arrive on another CTA's barrier (`bar` from map_to_cta).
+// Arrive on another CTA's barrier (`bar` from map_to_cta). Orders no memory between the CTAs: for handing
+// back tensor memory, after tc_fence_before.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // TMEM -> registers: each thread reads N consecutive 32-bit columns of its own lane.

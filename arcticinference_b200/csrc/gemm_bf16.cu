@@ -158,7 +158,23 @@ __device__ __forceinline__ void gelu8(float (&v)[8]) {
 
 // The epilogue of a tile whose output leaves in whole lines, one of eight warps: 32 rows from
 // warp_row0 on, alternate groups of 64 columns of the tile that starts at column b0.
+// EPI: what the epilogue does, known when it is compiled (the code of all options together did not stay in
+// the instruction cache), or kEpiAny: what the arguments say.
+enum Epilogue : int { kEpiAny = -1, kEpiScaled = 1, kEpiBias = 2, kEpiGelu = 4, kEpiResidual = 8, kEpiGated = 16 };
+
+template <int EPI>
 struct CoalescedTile {
+  static constexpr bool kAny = EPI < 0;
+  __device__ __forceinline__ static bool scaled(const GemmArgs& p) {
+    return kAny ? p.scale_a != nullptr : (EPI & kEpiScaled) != 0;
+  }
+  __device__ __forceinline__ static bool biased(const GemmArgs& p) {
+    return kAny ? p.bias != nullptr : (EPI & kEpiBias) != 0;
+  }
+  __device__ __forceinline__ static bool summed(const GemmArgs& p) {
+    return kAny ? p.residual != nullptr : (EPI & kEpiResidual) != 0;
+  }
+
   uint4 rq[8];
   // This lane's two of the group's 64 column factors or biases; they reach the other lanes through shared
   // memory. A load per eight columns from global memory, behind stores that might alias it, took
@@ -172,8 +188,8 @@ struct CoalescedTile {
       const long long c = b0 + c0 + lane + 32 * h;
       cv[h] = 0.f;
       if (c < p.rows_b) {
-        if (p.scale_a != nullptr) cv[h] = p.scale_b[c];
-        else if (p.bias != nullptr) cv[h] = __bfloat162float(p.bias[c]);
+        if (scaled(p)) cv[h] = p.scale_b[c];
+        else if (biased(p)) cv[h] = __bfloat162float(p.bias[c]);
       }
     }
   }
@@ -194,14 +210,13 @@ struct CoalescedTile {
   __device__ __forceinline__ void prefetch(const GemmArgs& p, long long warp_row0, long long b0, int half,
                                            int lane) {
     fetch_columns(p, b0, half * 64, lane);
-    if (p.residual != nullptr && half * 64 < p.bn) fetch_residual(p, warp_row0, b0, half * 64, lane);
+    if (summed(p) && half * 64 < p.bn) fetch_residual(p, warp_row0, b0, half * 64, lane);
   }
 
   // t_addr: the warp's lane quadrant of the accumulator; stg: its staging tile; cols: its 64 floats
   __device__ __forceinline__ void store(const GemmArgs& p, uint32_t t_addr, uint8_t* stg, float* cols,
                                         long long warp_row0, long long b0, int half, int lane, float sa) {
-    const bool scaled = p.scale_a != nullptr;
-    const bool add_rows = p.residual != nullptr;
+    const bool add_rows = summed(p);
     const bool row_ok = warp_row0 + lane < p.rows_a;
     // 64 output columns at a time: each thread converts its row, the warp transposes
     // through its private staging tile, and every store instruction then writes four
@@ -237,15 +252,15 @@ struct CoalescedTile {
           if (cj + 8 <= p.rows_b && c0 + 8 * j + 8 <= p.bn) {
             const float4 s0 = *reinterpret_cast<const float4*>(cols + 8 * j);
             const float4 s1 = *reinterpret_cast<const float4*>(cols + 8 * j + 4);
-            if (scaled) {
+            if (scaled(p)) {
               v[0] *= sa * s0.x; v[1] *= sa * s0.y; v[2] *= sa * s0.z; v[3] *= sa * s0.w;
               v[4] *= sa * s1.x; v[5] *= sa * s1.y; v[6] *= sa * s1.z; v[7] *= sa * s1.w;
-              if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
-            } else if (p.bias != nullptr) {
+              if (biased(p)) add8(v, *reinterpret_cast<const uint4*>(p.bias + cj));
+            } else if (biased(p)) {
               v[0] += s0.x; v[1] += s0.y; v[2] += s0.z; v[3] += s0.w;
               v[4] += s1.x; v[5] += s1.y; v[6] += s1.z; v[7] += s1.w;
             }
-            if (p.act == 1) gelu8(v);
+            if (kAny ? p.act == 1 : (EPI & kEpiGelu) != 0) gelu8(v);
             if (add_rows) add8(v, *at);
           }
           uint4 q;
@@ -259,7 +274,7 @@ struct CoalescedTile {
       __syncwarp();
       __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.out) + col;
       long long row_off = 0;
-      if (p.peer_cols > 0) {  // a 64-column group never straddles a destination
+      if (kAny && p.peer_cols > 0) {  // a 64-column group never straddles a destination
         base = p.peer_out[col / p.peer_cols] + col % p.peer_cols;
         row_off = p.peer_row_off;
       }
@@ -603,7 +618,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
       // The tile's column values and the residual's first columns are requested while the k-loop
       // runs: a lone tile per CTA pays for every load that waits for its accumulator.
       const long long warp_row0 = (long long)tile_a * kBlockM + quad * 32;
-      CoalescedTile ct;
+      CoalescedTile<kEpiAny> ct;
       if (p.coalesce) ct.prefetch(p, warp_row0, b0, half, lane);
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 400 + acc, w)) break;
       tc_fence_after();
@@ -849,6 +864,7 @@ __device__ __forceinline__ void decode_pair(const GemmArgs& p, int w, int& tile_
   tile_b = r / rows;
 }
 
+template <int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b, const GemmArgs p) {
@@ -914,7 +930,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         decode_pair(p, w, tile_a, tile_b);
         const int row_a = (2 * tile_a + rank) * kBlockM;
         // (gate / up: the even CTA stages gate rows, the odd one the same columns' up rows)
-        const int row_b = p.gate_rows > 0 ? tile_b * (int)half_b + rank * p.gate_rows
+        const int row_b = EPI == kEpiGated ? tile_b * (int)half_b + rank * p.gate_rows
                                           : tile_b * p.bn + rank * (int)half_b;
         for (int kb = 0; kb < p.kblocks_total; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, 100 + stage, kb)) {
@@ -1006,14 +1022,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const long long col0 = (long long)tile_b * p.bn;
       const float sa =
           (p.scale_a != nullptr && warp_row0 + lane < p.rows_a) ? p.scale_a[warp_row0 + lane] : 1.f;
-      CoalescedTile ct;
-      if (p.gate_rows == 0) ct.prefetch(p, warp_row0, col0, half, lane);
+      CoalescedTile<EPI> ct;
+      if (EPI != kEpiGated) ct.prefetch(p, warp_row0, col0, half, lane);
       if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 400 + acc, w)))
         break;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * 256u;
       uint8_t* stg = store_stage + (size_t)(warp - 2) * kStoreStageBytes;
-      if (p.gate_rows > 0)
+      if (EPI == kEpiGated)
         store_gated(p, t_addr, stg, warp_row0, tile_b, half, lane);
       else
         ct.store(p, t_addr, stg, column_values(store_stage, warp), warp_row0, col0, half, lane, sa);
@@ -1259,6 +1275,22 @@ static FewPlan few_plan_of(int M, int N, int kblocks, int group_max, int sms) {
   return plan;
 }
 
+// The pair kernel's forms with an epilogue of their own, and the one for any other.
+struct PairForm {
+  int epi;
+  void (*kernel)(CUtensorMap, CUtensorMap, GemmArgs);
+};
+static const PairForm pair_forms[] = {
+    {0, gemm_pair_kernel<0>},
+    {kEpiScaled, gemm_pair_kernel<kEpiScaled>},
+    {kEpiBias, gemm_pair_kernel<kEpiBias>},
+    {kEpiBias | kEpiGelu, gemm_pair_kernel<kEpiBias | kEpiGelu>},
+    {kEpiBias | kEpiResidual, gemm_pair_kernel<kEpiBias | kEpiResidual>},
+    {kEpiGated, gemm_pair_kernel<kEpiGated>},
+    {kEpiAny, gemm_pair_kernel<kEpiAny>},
+};
+constexpr int kPairForms = sizeof(pair_forms) / sizeof(pair_forms[0]);
+
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 32;
   while (p < v) p <<= 1;
@@ -1336,8 +1368,8 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   if (!attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    for (int i = 0; i < kPairForms && e == cudaSuccess; ++i)
+      e = cudaFuncSetAttribute(pair_forms[i].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(gemm_few_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
@@ -1572,7 +1604,13 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
       const long long tiles = (long long)a.tiles_a * a.tiles_b;
       const unsigned pairs = (unsigned)(tiles < sms / 2 ? tiles : sms / 2);
       const size_t smem = (size_t)a.stages * stage_bytes + 256 + kStoreBytes;
-      return launch_pdl_cluster(gemm_pair_kernel, dim3(2 * pairs), dim3(kGemmThreads), smem, stream, 2u,
+      const int epi = gate_rows > 0 ? kEpiGated
+                                    : (fp8 ? kEpiScaled : 0) | (bias != nullptr ? kEpiBias : 0) |
+                                          (act == 1 ? kEpiGelu : 0) | (residual != nullptr ? kEpiResidual : 0);
+      auto kernel = gemm_pair_kernel<kEpiAny>;
+      for (int i = 0; i < kPairForms; ++i)
+        if (pair_forms[i].epi == epi) kernel = pair_forms[i].kernel;
+      return launch_pdl_cluster(kernel, dim3(2 * pairs), dim3(kGemmThreads), smem, stream, 2u,
                                 ta, tb, a) == cudaSuccess
                  ? 0
                  : -5;

@@ -8,12 +8,13 @@
 // reaches accumulator rows that nobody reads. A stage is then little more than its weights, and the
 // ring keeps up to 200 KB of them in flight per SM. Two accumulators for more than 128 tokens. A stage
 // holds up to four k-blocks, each operand's fetched by one copy: a stage's wait, copies and commit
-// cost 0.17 us whatever its size, which with one block per stage was more than the block itself.
+// cost 0.25 us whatever its size, which with one block per stage was more than the block itself.
 //
 // Why a kernel of its own: the general one (gemm_bf16_kernel) stages 128 rows of tokens, and its long
 // code runs cold in a kernel of a few microseconds. 50 tokens, 768 x 768: 15.3 -> 4.7 us; 1 token,
 // 28672 x 4096 bf16 59.1 -> 41.6 us (5.6 of 6.46 TB/s), 4096 x 4096 14.1 -> 12.0; 128 tokens, 4096 x 14336
-// 38.9 -> 30.0; 128 tokens fp8, 4096 x 14336 26.0 -> 18.2; 256 tokens, 28672 x 4096 88.9 -> 58.9.
+// 38.9 -> 30.0; 128 tokens fp8, 4096 x 14336 26.0 -> 18.2; 256 tokens, 28672 x 4096 88.9 -> 58.9. With
+// programmatic launches 4.0, 40.3, 10.3, 28.7, 16.6 and 57.5.
 #pragma once
 
 namespace ab200 {
@@ -21,7 +22,7 @@ namespace ab200 {
 constexpr int kFewEpilogueWarps = 8;
 constexpr int kFewThreads = (2 + kFewEpilogueWarps) * 32;
 constexpr int kFewMaxStages = 32;
-constexpr int kFewHeader = 1024;   // barriers, in front of the stages
+constexpr int kFewHeader = 3072;   // barriers and the tile's column factors and biases, in front of the stages
 
 struct FewArgs {
   const float* scale_x;   // e4m3 operands: one factor per token and per feature
@@ -37,16 +38,21 @@ struct FewArgs {
   uint32_t tmem_cols;
 };
 
-// Eight finished columns from c on of a token's row.
-__device__ __forceinline__ void few_store8(const FewArgs& p, int m, int c, float (&v)[8]) {
+// Eight finished columns from c on of a token's row; `at`: the first one's place among `cols`, the factors
+// and, 256 floats on, the biases of the columns that this CTA finishes.
+__device__ __forceinline__ void few_store8(const FewArgs& p, int m, int c, const float* cols, int at, float sx,
+                                           float (&v)[8]) {
+  const float4* f = reinterpret_cast<const float4*>(cols + at);
   if (p.scale_x != nullptr) {
-    const float sx = p.scale_x[m];
-    const float4 s0 = *reinterpret_cast<const float4*>(p.scale_w + c);
-    const float4 s1 = *reinterpret_cast<const float4*>(p.scale_w + c + 4);
+    const float4 s0 = f[0], s1 = f[1];
     v[0] *= sx * s0.x; v[1] *= sx * s0.y; v[2] *= sx * s0.z; v[3] *= sx * s0.w;
     v[4] *= sx * s1.x; v[5] *= sx * s1.y; v[6] *= sx * s1.z; v[7] *= sx * s1.w;
   }
-  if (p.bias != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.bias + c));
+  if (p.bias != nullptr) {
+    const float4 b0 = f[64], b1 = f[65];
+    v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+    v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
+  }
   if (p.act == 1) gelu8(v);
   if (p.residual != nullptr) add8(v, *reinterpret_cast<const uint4*>(p.residual + m * p.ldr + c));
   uint4 q;
@@ -85,6 +91,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   const uint32_t done_bar = base + 8u * (2 * kFewMaxStages);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (base - raw) + 8 * (2 * kFewMaxStages + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  float* cols = reinterpret_cast<float*>(smem_raw + (base - raw) + 1024);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -189,6 +197,15 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     }
   } else {
     pdl_wait();
+    // Factors and biases of the columns come from memory while the products run: a load per eight columns
+    // after them cost an epilogue several trips to memory, one after the other.
+    const int t = (int)threadIdx.x - 64, width = p.bn / p.splits;
+    const int c = tile * p.bn + split * width + t;
+    if (t < width && c < p.N) {
+      if (p.scale_x != nullptr) cols[t] = p.scale_w[c];
+      if (p.bias != nullptr) cols[256 + t] = __bfloat162float(p.bias[c]);
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kFewEpilogueWarps * 32) : "memory");
     ok = __all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, p.status, 400, n));
     tc_fence_after();
   }
@@ -198,6 +215,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     if (warp >= 2 && ok) {
       for (int m0 = quad * 32; m0 < p.M; m0 += 128) {
         const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (m0 >= 128 ? (uint32_t)p.bn : 0u);
+        const float sx = p.scale_x != nullptr && m0 + lane < p.M ? p.scale_x[m0 + lane] : 1.f;
 #pragma unroll 1
         for (int c0 = part * 16; c0 < p.bn; c0 += 32) {
           uint32_t r[16];
@@ -209,7 +227,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
             float v[8];
 #pragma unroll
             for (int t = 0; t < 8; ++t) v[t] = __uint_as_float(r[8 * g + t]);
-            if (m0 + lane < p.M && c < p.N) few_store8(p, m0 + lane, c, v);
+            if (m0 + lane < p.M && c < p.N) few_store8(p, m0 + lane, c, cols, c0 + 8 * g, sx, v);
           }
           __syncwarp();
         }
@@ -257,7 +275,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
           v[0] += lo.x; v[1] += lo.y; v[2] += lo.z; v[3] += lo.w;
           v[4] += hi.x; v[5] += hi.y; v[6] += hi.z; v[7] += hi.w;
         }
-        few_store8(p, m, c, v);
+        few_store8(p, m, c, cols, c8, p.scale_x != nullptr ? p.scale_x[m] : 1.f, v);
       }
     }
   }
@@ -291,10 +309,10 @@ static int few_stages(int M, int x_rows, int bn, int splits, int group, int most
 
 // Width of the tiles, K splits and k-blocks per stage: few enough to try them all. Times in us, fitted to a
 // sweep over all plans of the projections of 768- and 4096-wide models with 1 - 256 tokens: weights come
-// from HBM at 6.4 MB/us in all; an SM takes in weights and tokens at 0.1 MB/us; a stage costs its
-// wait, copies and commit (0.17), a block its four instructions (44 cycles or half a cycle per
-// feature each); a cluster's exchange 2 and 0.06 per KB of a CTA's sums. `group_max` is 1 where K ends
-// inside a block.
+// from HBM at 6.4 MB/us in all; an SM takes in weights and tokens at 0.2 MB/us; a stage costs its
+// wait, copies and commit (0.25), a block its four instructions (44 cycles or half a cycle per
+// feature each); a cluster's exchange 1.5 and 0.09 per KB of a CTA's sums. `group_max` is 1 where K
+// ends inside a block.
 static FewPlan plan_few(int M, int N, int kblocks, int group_max, int sms, int (*capacity)(int, size_t)) {
   FewPlan best = {0, 0, 0, 0, 0};
   double best_t = 1e30;
@@ -315,13 +333,13 @@ static FewPlan plan_few(int M, int N, int kblocks, int group_max, int sms, int (
         const int cap = splits > 1 ? capacity(splits, 226 * 1024) * splits : sms;
         if (cap <= 0) continue;
         const double waves = (double)((tiles * splits + cap - 1) / cap);
-        const double sm_us = (bn + x_rows) * group * 128.0 / 0.1e6;
-        const double mma_us = 0.17 + group * 4.0 * halves * (bn > 88 ? bn / 2.0 : 44.0) / 1.9e3;
+        const double sm_us = (bn + x_rows) * group * 128.0 / 0.2e6;
+        const double mma_us = 0.25 + group * 4.0 * halves * (bn > 88 ? bn / 2.0 : 44.0) / 1.9e3;
         const double hbm_us = (double)N * kblocks * 128.0 / 6.4e6;
         double t = waves * (per * (sm_us > mma_us ? sm_us : mma_us) + 0.05 * halves * bn / 16 / splits);
         if (t < hbm_us) t = hbm_us + 0.1 * t;
         t += 4.0 * (waves - 1.0);
-        if (splits > 1) t += 2.0 + 0.06 * M * bn * 4.0 / 1024.0;
+        if (splits > 1) t += 1.5 + 0.09 * M * bn * 4.0 / 1024.0;
         if (t < best_t - 0.05) {
           best_t = t;
           best = {bn, splits, group, stages, smem};

@@ -1191,6 +1191,14 @@ static int pick_stages(int bn) {
   return s;
 }
 
+static bool cluster_splits_off() {
+  static const bool off = [] {
+    const char* e = getenv("AB200_GEMM_CLUSTER");
+    return e != nullptr && e[0] == '0';
+  }();
+  return off;
+}
+
 // How many clusters of `cs` CTAs (one CTA per SM: the kernel takes an SM's shared memory) the
 // device can hold at once; 0 when such a cluster cannot be placed.
 static int cluster_capacity(int cs, size_t smem) {
@@ -1262,14 +1270,19 @@ static int pick_tile_width(int tiles_a, int N, int kblocks, int units, bool pair
 }
 
 // The plan of a size, made once (a hundred candidates cost the host 2 us, as much as the launch).
-static FewPlan few_plan_of(int M, int N, int kblocks, int group_max, int sms) {
+// Token counts are planned in classes, so that a step and the same step padded to a captured one's size
+// sum in the same order.
+static FewPlan few_plan_of(int tokens, int N, int kblocks, int group_max, int sms) {
+  int M = 8;
+  while (M < tokens) M += M < 128 ? M : 64;
   static std::mutex mu;
   static std::unordered_map<uint64_t, FewPlan> plans;
   const uint64_t key = ((uint64_t)M << 54) ^ ((uint64_t)group_max << 50) ^ ((uint64_t)N << 20) ^ (uint64_t)kblocks;
   std::lock_guard<std::mutex> lock(mu);
   auto it = plans.find(key);
   if (it != plans.end()) return it->second;
-  const FewPlan plan = plan_few(M, N, kblocks, group_max, sms, cluster_capacity);
+  const FewPlan plan = plan_few(M, N, kblocks, group_max, sms,
+                                cluster_splits_off() ? [](int, size_t) { return 0; } : cluster_capacity);
   if (plans.size() > 8192) plans.clear();
   plans.emplace(key, plan);
   return plan;
@@ -1529,11 +1542,7 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   // One row of tiles (at most 128 tokens): consider splitting K inside thread-block clusters
   // instead of through the workspace. The scatter epilogue qualifies too: the CTA that
   // finishes a column range stores it to the rank that owns it.
-  static const bool cluster_off = [] {
-    const char* e = getenv("AB200_GEMM_CLUSTER");
-    return e != nullptr && e[0] == '0';
-  }();
-  if (!a.transposed && a.tiles_a == 1 && !cluster_off && (force_splits == 0 || peer_cols > 0) &&
+  if (!a.transposed && a.tiles_a == 1 && !cluster_splits_off() && (force_splits == 0 || peer_cols > 0) &&
       N % 8 == 0 && ldo % 8 == 0 && (peer_cols == 0 || peer_cols % 8 == 0) &&
       (reinterpret_cast<uintptr_t>(bias) % 16) == 0 && (residual == nullptr || ldr % 8 == 0)) {
     double best = plan_cost_us(a.tiles_b, a.splits, a.kblocks_total, sms, false, M, N);

@@ -8,6 +8,8 @@
 // The reference obtains these from the vLLM pooling model that its embedding replica wraps
 // (arctic_inference/embedding/replica.py:83-128).
 
+#include <string.h>
+
 #include "api.h"
 #include "common/pdl.cuh"
 #include "common/ptx.cuh"
@@ -372,10 +374,30 @@ int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void*
   const float scale = 1.f / sqrtf((float)D);
   char* qkv = reinterpret_cast<char*>(wide);
   const size_t part = (size_t)hidden * 2;   // bytes
+  auto linear = [&](const void* in, const void* w, const void* bias, void* out, int n, int k, int act,
+                    const void* residual) -> int {
+    Ab200LinearDesc d;
+    memset(&d, 0, sizeof(d));
+    d.x = in;
+    d.ldx = k;
+    d.w = w;
+    d.ldw = k;
+    d.out = out;
+    d.ldo = n;
+    d.M = T;
+    d.N = n;
+    d.K = k;
+    d.bias = bias;
+    d.residual = residual;
+    d.ldr = residual != nullptr ? n : 0;
+    d.act = act;
+    d.status = status;
+    d.w_static = 1;   // parameters: nothing enqueued here writes them
+    return ab200_linear_desc(&d, stream);
+  };
   for (int l = 0; l < n_layers; ++l) {
     const Ab200BertLayer& w = layers[l];
-    int rc = ab200_linear_bf16(h, hidden, w.wqkv, hidden, wide, 3 * hidden, T, 3 * hidden, hidden, w.bqkv,
-                               nullptr, 0, 0, nullptr, 0, 0, status, stream);
+    int rc = linear(h, w.wqkv, w.bqkv, wide, 3 * hidden, hidden, 0, nullptr);
     if (rc != 0) return rc;
     rc = D == kShortDim && max_len <= kShortLen
              ? ab200_attention_short(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, work, num_work,
@@ -383,19 +405,11 @@ int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void*
              : ab200_attention(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, T, 0, nullptr, 0, work,
                                num_work, nullptr, 1, T, heads, heads, D, 0, scale, a, hidden, nullptr, nullptr,
                                nullptr, tile_keys, status, stream);
-    if (rc != 0) return rc;
-    rc = ab200_linear_bf16(a, hidden, w.wo, hidden, x, hidden, T, hidden, hidden, w.bo, h, hidden, 0,
-                           nullptr, 0, 0, status, stream);
-    if (rc != 0) return rc;
-    rc = ab200_layernorm(x, nullptr, w.ln1_g, w.ln1_b, h, T, hidden, eps, stream);
-    if (rc != 0) return rc;
-    rc = ab200_linear_bf16(h, hidden, w.wi, hidden, wide, inter, T, inter, hidden, w.bi, nullptr, 0, 1,
-                           nullptr, 0, 0, status, stream);
-    if (rc != 0) return rc;
-    rc = ab200_linear_bf16(wide, inter, w.wd, inter, x, hidden, T, hidden, inter, w.bd, h, hidden, 0,
-                           nullptr, 0, 0, status, stream);
-    if (rc != 0) return rc;
-    rc = ab200_layernorm(x, nullptr, w.ln2_g, w.ln2_b, h, T, hidden, eps, stream);
+    if (rc == 0) rc = linear(a, w.wo, w.bo, x, hidden, hidden, 0, h);
+    if (rc == 0) rc = ab200_layernorm(x, nullptr, w.ln1_g, w.ln1_b, h, T, hidden, eps, stream);
+    if (rc == 0) rc = linear(h, w.wi, w.bi, wide, inter, hidden, 1, nullptr);
+    if (rc == 0) rc = linear(wide, w.wd, w.bd, x, hidden, inter, 0, h);
+    if (rc == 0) rc = ab200_layernorm(x, nullptr, w.ln2_g, w.ln2_b, h, T, hidden, eps, stream);
     if (rc != 0) return rc;
   }
   return 0;

@@ -26,7 +26,7 @@ environment_variables: dict[str, Callable[[], Any]] = {
     # ---- tuning switches of the kernel library and the communicator (docs/kernels.md,
     # docs/parallelism.md); each names the default in its second argument
     # programmatic dependent launch of the serving kernels (read once by the kernel library)
-    "AB200_PDL": _flag("AB200_PDL", "0"),
+    "AB200_PDL": _flag("AB200_PDL", "1" if os.getenv("WORLD_SIZE", "1") in ("", "0", "1") else "0"),
     # split-K of one-row-of-tiles GEMMs inside thread-block clusters (0: through the workspace)
     "AB200_GEMM_CLUSTER": _flag("AB200_GEMM_CLUSTER", "1"),
     # fp8 codes stored in 16-row x 128-byte tiles instead of row-major

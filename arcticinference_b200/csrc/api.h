@@ -307,7 +307,7 @@ int ab200_latent_rope_cache(void* q, const void* ckv, long long ld, const void* 
 // ---- moe.cu
 int ab200_moe_route(const void* x, int x_dtype, const void* w, const void* b, long long T, int W, int E,
                     int experts, int top, int mode, float scale, int groups, int keep, void* ids,
-                    void* weights, void* state, void* cursor, void* tiles, void* num_tiles, int dtype,
+                    void* weights, void* state, void* cursor, void* tiles, void* num_tiles, int even, int dtype,
                     cudaStream_t stream);
 int ab200_moe_permute(const void* x, const void* ids, void* cursor, void* rows, void* xp,
                       long long T, int W, int top, int experts, int dtype, cudaStream_t stream);
@@ -342,7 +342,7 @@ int ab200_grouped_gemm(const void* x, long long ldx, long long x_gstride, long l
                        const void* w, long long ldw, long long w_gstride, void* out, long long ldo,
                        long long out_gstride, int M, int N, int K, int groups, const void* tiles,
                        const void* num_tiles, int max_tiles, int act, float act_limit,
-                       float act_alpha, int* status, cudaStream_t stream);
+                       float act_alpha, int pairs, int* status, cudaStream_t stream);
 
 // ---- latent_attention.cu
 int ab200_latent_attention(const void* q, long long q_rows, const void* cache, int num_blocks,

@@ -340,6 +340,14 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* 
       ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const void* tmap, uint32_t bar,
+                                                 int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
 // Arrive on another CTA's barrier (`bar` from map_to_cta). Orders no memory between the CTAs: for handing
 // back tensor memory, after tc_fence_before.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {

@@ -66,6 +66,7 @@ struct RouteArgs {
   int* cursor;         // [E] first row of each expert
   int4* tiles;
   int* num_tiles;
+  int even;            // an even number of tiles per expert, the last one empty if need be
 };
 
 // Run by the last block: counts -> first rows and tiles; leaves the counts at zero.
@@ -84,7 +85,8 @@ __device__ void moe_plan(const RouteArgs& p, int* sh) {
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int e = e0 + threadIdx.x;
       const int c = e < E ? count[e] : 0;
-      const int k = (c + kTileRows - 1) / kTileRows;
+      int k = (c + kTileRows - 1) / kTileRows;
+      if (p.even) k = (k + 1) / 2 * 2;
       int rs = c, ts = k;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -107,8 +109,10 @@ __device__ void moe_plan(const RouteArgs& p, int* sh) {
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     p.cursor[e] = first[e];
-    for (int r = 0, k = 0; r < count[e]; r += kTileRows, ++k)
+    int k = 0;
+    for (int r = 0; r < count[e]; r += kTileRows, ++k)
       p.tiles[tile0[e] + k] = make_int4(e, first[e] + r, min(kTileRows, count[e] - r), 0);
+    if (p.even && (k & 1)) p.tiles[tile0[e] + k] = make_int4(e, first[e], 0, 0);
   }
 }
 
@@ -373,11 +377,11 @@ extern "C" {
 // null; the first `experts` of the E outputs are experts, the others the identity; mode, scale, groups,
 // keep: see RouteArgs. ids int32 and weights fp32
 // [T, top]; state int32 [experts + 1], zero; cursor int32 [experts]; tiles int32 x 4 [T * top / 128 +
-// experts at most]; num_tiles int32 [1]
+// experts at most, twice the experts with `even`]; num_tiles int32 [1]; even: see RouteArgs
 int ab200_moe_route(const void* x, int x_dtype, const void* w, const void* b, long long T, int W, int E,
                     int experts, int top, int mode, float scale, int groups, int keep, void* ids,
-                    void* weights, void* state, void* cursor, void* tiles, void* num_tiles, int dtype,
-                    cudaStream_t stream) {
+                    void* weights, void* state, void* cursor, void* tiles, void* num_tiles, int even,
+                    int dtype, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (top < 1 || top > E || experts < 1 || experts > E) return -2;
   if (mode < kRouteChosen || mode > kRouteSigmoid || (x_dtype != 1 && x_dtype != dtype)) return -2;
@@ -404,6 +408,7 @@ int ab200_moe_route(const void* x, int x_dtype, const void* w, const void* b, lo
   a.cursor = reinterpret_cast<int*>(cursor);
   a.tiles = reinterpret_cast<int4*>(tiles);
   a.num_tiles = reinterpret_cast<int*>(num_tiles);
+  a.even = even;
   // many tokens: several per block, so that the router's weights are read less often
   const bool wide = T >= 148 * 8 && (size_t)8 * (W + E) * 4 <= 110 * 1024;
   if (dtype == 0) return wide ? launch_route<bf16, 8>(a, stream) : launch_route<bf16, 1>(a, stream);

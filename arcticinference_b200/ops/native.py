@@ -151,10 +151,10 @@ def _declare(L: ctypes.CDLL) -> None:
                                       P, P]),
         "ab200_latent_rope_cache": (I, [P, P, LL, P, I, P, P, P, LL, I, I, I, I, I, I, LL, F, I, P,
                                         P]),
-        "ab200_moe_route": (I, [P, I, P, P, LL, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, P]),
+        "ab200_moe_route": (I, [P, I, P, P, LL, I, I, I, I, I, F, I, I, P, P, P, P, P, P, I, I, P]),
         "ab200_moe_permute": (I, [P, P, P, P, P, LL, I, I, I, I, P]),
         "ab200_grouped_gemm": (I, [P, LL, LL, LL, P, LL, LL, P, LL, LL, I, I, I, I, P, P, I, I, F,
-                                   F, P, P]),
+                                   F, I, P, P]),
         "ab200_latent_attention": (I, [P, LL, P, I, I, P, I, P, I, P, I, LL, I, I, I, I, I, I, F, P, P,
                                        LL, P, P, P, P, P]),
         "ab200_attention_ext": (I, [P, LL, P, P, LL, LL, I, P, I, P, I, P, I, LL, I, I, I, I, I, I, P,

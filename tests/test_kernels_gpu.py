@@ -468,6 +468,32 @@ def test_attention_merge_pieces(T, ns):
     _close(out, ref.attention(q, kc, vc, bt, q_lens, kv_lens, Hq, Hkv, D, 1 / math.sqrt(D)), 2e-2, 2e-2)
 
 
+# experts on pairs of tiles: odd and even numbers of tiles, an expert without rows, K and N that end inside a
+# block and a tile
+@pytest.mark.parametrize("N,K", [(512, 256), (800, 136)])
+@pytest.mark.parametrize("act", [None, "silu"])
+def test_grouped_linear_pairs(N, K, act):
+    from arcticinference_b200.ops import stream_ops as st
+    T, E, top = 3001, 6, 3
+    x, router, b = _rand(T, K), _rand(E, K, scale=0.1), torch.zeros(E, device=DEV)
+    b[2], b[4] = -100.0, 1.0
+    r, rows = st.route(x, x, router, b, top)
+    assert r.even
+    w = _rand(E, N, K, scale=1.0 / math.sqrt(K))
+    out = st.grouped_linear(rows, w, r, act=act)
+    ops.check_status()
+    expert = torch.empty(T * top, dtype=torch.long, device=DEV)
+    expert[r.rows.long().reshape(-1)] = r.ids.long().reshape(-1)
+    z = torch.zeros(T * top, N, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        z[expert == e] = rows[expert == e].double() @ w[e].double().t()
+    if act:
+        g, u = (t.flatten(1) for t in z.view(T * top, N // 32, 2, 16).unbind(2))
+        z = torch.nn.functional.silu(g) * u
+    # one rounding to bf16; fp32 sums and the fast exponential before it
+    assert ((out.double() - z).abs() <= z.abs() * 2.0 ** -8 + 2e-4).all()
+
+
 @pytest.mark.parametrize("H,D,seq_lens", [(12, 64, [50, 128, 3, 512]), (4, 128, [77, 300])])
 def test_encoder_attention(H, D, seq_lens):
     T = sum(seq_lens)

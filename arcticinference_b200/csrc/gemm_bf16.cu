@@ -1322,11 +1322,10 @@ size_t ab200_linear_bf16_workspace_bytes(int M, int N, int K) {
   return (size_t)(M <= 128 ? 16 : 8) * (size_t)M * (size_t)N * sizeof(float);
 }
 
-// One tcgen05.mma (cta_group::1) is accepted every ~186 SM cycles whatever its shape
-// (measured on B200 for M = 64/128, N = 16..256, bf16 and fp8), so a k-loop is bound by its
-// instruction count unless every instruction carries enough work. With few tokens the
-// weights therefore go on the N side, 256 features per instruction, and the tokens on the
-// (padded) M side; split-K then spreads the instructions over all SMs.
+// For the calls with few tokens that the general kernel still serves (scattered outputs, ordering between
+// ranks): the weights go on the N side, 256 features per instruction, the tokens on the (padded) M side, and
+// split-K spreads the instructions over all SMs. The interval is that of instructions issued from a branch of one
+// thread; the warp-uniform loop takes 64 to 128 cycles, so these plans err towards more splits.
 constexpr double kMmaIssueCycles = 186.0;
 
 // Split-K factor for a one-row-of-tiles (M <= 128) token-major GEMM: the smallest estimate of

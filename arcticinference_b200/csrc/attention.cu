@@ -169,8 +169,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   // launch): barrier and TMEM set-up and the clearing of the K/V stages below overlap its
   // tail. The work list is uploaded by the host before the step's first kernel and is the
   // only global memory read ahead of pdl_wait(); nothing is written before it.
-  pdl_trigger();
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_trigger();
     pdl_wait();
     if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
     tail_signal(p.sig, total_blocks);
@@ -209,6 +209,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int q_tok0 = wk[1];
   const int n_q_tok = wk[2];
   if (n_q_tok <= 0) {  // padding entry of a fixed-size work list
+    pdl_trigger();
     pdl_wait();
     tail_signal(p.sig, total_blocks);
     return;
@@ -265,6 +266,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();   // (tensor memory is owned)
   pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base;           // S buffers at columns 0, TK
@@ -770,8 +772,8 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   const unsigned int total_blocks = gridDim.x;
-  pdl_trigger();
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_trigger();
     pdl_wait();
     if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
     tail_signal(p.sig, total_blocks);
@@ -801,6 +803,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const int q_tok0 = wk[1];
   const int n_q_tok = wk[2];
   if (n_q_tok <= 0) {  // padding entry of a fixed-size work list
+    pdl_trigger();
     pdl_wait();
     tail_signal(p.sig, total_blocks);
     return;
@@ -860,6 +863,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();   // (tensor memory is owned)
   pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   // S (and P over it) of tile t at columns 128 t, O at 256 + D t

@@ -100,7 +100,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   constexpr int kElems = FP8 ? kBlockKFp8 : kBlockK;
   const int g0 = split * p.groups_per_split;
   const int n = min(p.groups_per_split, p.groups - g0);
-  pdl_trigger();
   if (warp == 0 && lane == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -125,6 +124,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();   // (tensor memory is owned)
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
 

@@ -4,12 +4,19 @@
 // writes are visible; what comes before the wait (barrier and TMEM set-up, tensor-map
 // prefetch, loads of weights that no kernel writes) overlaps the earlier kernel's tail, and
 // the launch latency disappears behind it. `pdl_trigger()` tells the scheduler that the next
-// kernel of the stream may be placed; it is issued as early as possible because the next
+// kernel of the stream may be placed; it is issued as early as the rules allow because the next
 // kernel protects itself with its own wait.
 //
 // Rules every kernel launched through `launch_pdl` follows:
-//   * no global write and no read of data another kernel produces before `pdl_wait()`;
-//   * every thread that touches such data executes `pdl_wait()` first.
+//   * no global write and no read of data another kernel produces before `pdl_wait()`. What a copy of the
+//     host's has written ahead of the step's first kernel (an attention work list) and parameters may be
+//     read: copies signal nothing early, so no kernel after one starts before it is done. A kernel of
+//     this library must not write either: a kernel two places further on could read too soon;
+//   * every thread that touches such data executes `pdl_wait()` first, and no block leaves before one of its
+//     threads has (a kernel that has finished says that those before it have);
+//   * `pdl_trigger()` comes behind the barrier that follows `tcgen05.alloc`. The allocation waits without a
+//     limit. A block of the next kernel that shares the SM could otherwise take the columns first and then
+//     wait for this kernel, which waits for them.
 // A kernel launched without the attribute sees both instructions as no-ops, and a kernel
 // launched with a plain <<<>>> after one of these waits for its full completion as usual.
 #pragma once

@@ -363,6 +363,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
     return;
   }
@@ -381,9 +383,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-
-  // the next kernel of the stream may be placed as SMs free up; it waits for this one itself
-  pdl_trigger();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -406,6 +405,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // the next kernel of the stream may be placed as SMs free up; it waits for this one itself
+  pdl_trigger();   // (tensor memory is owned)
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t acc_stride = p.tmem_cols / 2;
 
@@ -871,6 +872,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 900, (int)(smem_u32(smem) & 1023u));
     return;
   }
@@ -891,7 +894,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -914,6 +916,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   cluster_sync();   // the other CTA's barriers are ready for this one's copies and arrivals
   tc_fence_after();
+  pdl_trigger();   // (tensor memory is owned)
   const uint32_t tmem_base = *tmem_slot;
 
   const int total_work = p.tiles_a * p.tiles_b;

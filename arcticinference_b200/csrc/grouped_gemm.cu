@@ -141,7 +141,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -166,6 +165,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t acc_stride = p.tmem_cols / 2;
+  pdl_trigger();   // (tensor memory is owned)
   pdl_wait();   // the tile list and the activations come from earlier kernels
   const int m_total = p.tiles != nullptr ? *p.num_tiles : p.groups * p.m_tiles;
   const int total_work = m_total * p.n_tiles;
@@ -299,6 +299,8 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   extern __shared__ __align__(1024) uint8_t pair_smem[];
   uint8_t* smem = pair_smem;
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need 1024-byte alignment
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) report_error(p.status, kErrBadArgument, 1100, (int)(smem_u32(smem) & 1023u));
     return;
   }
@@ -317,7 +319,6 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   const int lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
 
-  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full_bar(s), 1);
@@ -341,6 +342,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   cluster_sync();   // the other CTA's barriers are ready for this one's copies and arrivals
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // (tensor memory is owned)
   pdl_wait();   // the tile list and the activations come from earlier kernels
   const int total_work = *p.num_tiles / 2 * p.n_tiles;
   const int first_work = (int)blockIdx.x / 2, work_step = (int)gridDim.x / 2;

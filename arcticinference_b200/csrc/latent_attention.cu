@@ -134,10 +134,10 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  pdl_trigger();
   const int* wk = p.work + (long long)blockIdx.x * 8;
   const int n_rows = wk[2];
   if (n_rows <= 0) {   // padding entry of a fixed-size work list
+    pdl_trigger();
     pdl_wait();
     return;
   }
@@ -194,6 +194,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();   // (tensor memory is owned)
   pdl_wait();
   const uint32_t tS = tmem_slot;                 // S buffers at columns 0, NR
   const uint32_t tO = tmem_slot + 2 * NR;        // R / 128 blocks of NR columns

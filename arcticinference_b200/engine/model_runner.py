@@ -386,7 +386,7 @@ class ModelRunner:
                 bt_sel = bt_t[ops.upload(np.asarray(keep, dtype=np.int64), dev)].contiguous() \
                     if len(keep) != bt_t.shape[0] else bt_t
                 batch.sel_attn_meta = ops.build_attention_metadata(sq, skv, bt_sel, self.G, m.h,
-                                                                   m.D, dev, Hkv=m.hkv)
+                                                                   m.D, dev, Hkv=m.hkv, block_size=bs)
         return batch, rows
 
     # ---------------------------------------------------------------- sampling

@@ -242,7 +242,7 @@ class LlamaModel:
         """The step's attention description, ``ForwardBatch.attn_meta``."""
         return ops.build_attention_metadata(q_lens, kv_lens, block_tables, self.h // self.hkv,
                                             self.h, self.D, self.device, Hkv=self.hkv,
-                                            wide=True)
+                                            wide=True, block_size=block_size)
 
     def decode_plans(self, bucket: int, max_q: int, block_size: int) -> list:
         """What a captured decode step of ``bucket`` tokens plans per step: one entry per kind

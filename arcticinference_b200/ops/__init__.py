@@ -858,7 +858,7 @@ def decode_splits(ctas: int, key_tiles: int, slots: int, most: int = 16) -> int:
 def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: int = 148,
                         Hkv: int = 1, seq_rows=None, allow_split: bool = True,
                         max_splits_cap: int = 16, mask=None, align: int = 1, rows_per_item: int = 128,
-                        fill_slots: bool = False):
+                        fill_slots: bool = False, slots: int | None = None):
     """Pure-host planner. Returns (work [n,8] int32 ndarray, tok_splits [T] int32, max_splits).
     ``mask`` (a MaskSpec): a tile's keys start at the first one its rows see, rounded down to a
     multiple of ``align`` (the cache's block size).
@@ -868,10 +868,13 @@ def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: i
     tiles to occupy the GPU (decode), the keys of each sequence are cut into up to 16 splits
     of whole 128-key tiles; with ``fill_slots`` (calls of the 64-key
     kernel, whatever padding they carry) the number follows from how CTAs of the decode
-    kernel share the SMs (:func:`decode_splits`)."""
+    kernel share the SMs (:func:`decode_splits`). ``slots``: the CTAs of the call's kernel that the GPU holds
+    at a time (:func:`attention_slots`); without it, two per SM for decode-shaped calls."""
     tpt = rows_per_item // G
+    if slots is None:
+        slots = num_sms * (2 if fill_slots or q_lens and max(q_lens) * G <= 32 else 1)
     if len(q_lens) >= 16 and max(q_lens) == 1 and min(q_lens) == 1:
-        return _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split,
+        return _plan_decode_work(kv_lens, G, causal, slots, Hkv, seq_rows, allow_split,
                                  max_splits_cap, mask, align, fill_slots)
     first = (lambda pos: 0) if mask is None else \
         (lambda pos: int(mask.first_key(pos)) // align * align)
@@ -879,8 +882,6 @@ def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: i
     T = int(sum(q_lens))
     tok_splits = np.ones(max(T, 1), dtype=np.int32)
     n_tiles_total = sum((ql + tpt - 1) // tpt for ql in q_lens)
-    if fill_slots or q_lens and max(q_lens) * G <= 32:
-        num_sms *= 2  # decode-shaped calls run two CTAs per SM (64-key tiles)
     t0 = 0
     max_splits = 1
     for i, (ql, kl) in enumerate(zip(q_lens, kv_lens)):
@@ -890,10 +891,10 @@ def plan_attention_work(q_lens, kv_lens, G: int, causal: bool = True, num_sms: i
         lo = first(kl - ql)
         key_tiles = (kl - lo + TILE_KEYS - 1) // TILE_KEYS
         ns = 1
-        if allow_split and n_tiles_total * Hkv < num_sms and key_tiles > 4:
-            want = max(1, num_sms // max(1, n_tiles_total * Hkv))
+        if allow_split and n_tiles_total * Hkv < slots and key_tiles > 4:
+            want = max(1, slots // max(1, n_tiles_total * Hkv))
             if fill_slots:
-                want = decode_splits(n_tiles_total * Hkv, key_tiles, num_sms, int(min(16, max_splits_cap)))
+                want = decode_splits(n_tiles_total * Hkv, key_tiles, slots, int(min(16, max_splits_cap)))
             ns = int(min(16, max_splits_cap, want, max(1, key_tiles // 2)))
         tiles_per_split = (key_tiles + ns - 1) // ns
         ns = (key_tiles + tiles_per_split - 1) // tiles_per_split
@@ -933,25 +934,23 @@ def tail_split_plan(n_seqs: int, Hkv: int, slots: int, max_splits: int = 4):
     return -(-rem // Hkv), pieces
 
 
-def _plan_decode_work(kv_lens, G, causal, num_sms, Hkv, seq_rows, allow_split, max_splits_cap,
+def _plan_decode_work(kv_lens, G, causal, slots, Hkv, seq_rows, allow_split, max_splits_cap,
                       mask=None, align=1, fill_slots=False):
     """The planner above for the one-token-per-sequence case, on arrays (same rows, same
     order): a serving step with a thousand sequences must not spend milliseconds here."""
     kl = np.asarray(kv_lens, dtype=np.int64)
     R = kl.size
-    if G <= 32:
-        num_sms *= 2
     lo = np.zeros_like(kl) if mask is None else mask.first_key(kl - 1) // align * align
     key_tiles = (kl - lo + TILE_KEYS - 1) // TILE_KEYS
     ns = np.ones(R, dtype=np.int64)
-    if allow_split and R * Hkv < num_sms:
-        want = max(1, num_sms // max(1, R * Hkv))
-        if G <= 32 and fill_slots:
-            want = decode_splits(R * Hkv, int(key_tiles.mean()), num_sms, int(min(16, max_splits_cap)))
+    if allow_split and R * Hkv < slots:
+        want = max(1, slots // max(1, R * Hkv))
+        if fill_slots:
+            want = decode_splits(R * Hkv, int(key_tiles.mean()), slots, int(min(16, max_splits_cap)))
         cand = np.minimum(np.minimum(16, max_splits_cap), np.minimum(want, np.maximum(1, key_tiles // 2)))
         ns = np.where(key_tiles > 4, cand, 1)
     elif allow_split and max_splits_cap > 1:
-        n_cut, pieces = tail_split_plan(R, Hkv, num_sms, int(min(4, max_splits_cap)))
+        n_cut, pieces = tail_split_plan(R, Hkv, slots, int(min(4, max_splits_cap)))
         if n_cut > 0:
             # the longest sequences are cut (at least 4 tiles per piece)
             longest = np.argsort(-(kl - lo), kind="stable")[:n_cut]
@@ -985,9 +984,15 @@ def upload(a: np.ndarray, device) -> torch.Tensor:
     return t.to(dev, non_blocking=True)
 
 
-def pick_tile_keys(q_lens, G: int) -> int:
-    """64-key tiles when every sequence's query rows fit one warp of the 128-row tile."""
-    return 64 if q_lens and max(q_lens) * G <= 32 else 128
+def pick_tile_keys(q_lens, G: int, block_size: int = 0) -> int:
+    """64-key tiles when every sequence's query rows fit one warp of the 128-row tile and a block of the
+    cache fits a tile."""
+    return 64 if q_lens and max(q_lens) * G <= 32 and block_size <= 64 else 128
+
+
+def attention_slots(tile_keys: int, num_sms: int = 148) -> int:
+    """CTAs that the GPU holds at a time: two per SM of the 64-key kernel, one of any other."""
+    return num_sms * (2 if tile_keys == 64 else 1)
 
 
 SHORT_TOKENS = 128   # longest sequence of the kernel for many short ones
@@ -1010,16 +1015,19 @@ def wide_tiles_pay(q_lens, G: int, Hkv: int, D: int, num_sms: int = 148) -> bool
 def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, causal=True,
                              Hkv=None, seq_rows=None, allow_split=True,
                              work_capacity: int | None = None, mask=None,
-                             align: int = 1, wide: bool = False) -> AttentionMetadata:
+                             align: int = 1, wide: bool = False, block_size: int = 0) -> AttentionMetadata:
     """``wide``: the calls that will use this plan take either arrangement of rows
-    (:func:`attention`, :func:`attention_contiguous`), so the better one may be chosen."""
+    (:func:`attention`, :func:`attention_contiguous`), so the better one may be chosen. ``block_size``: the
+    paged cache's, which decides on the kernel (:func:`pick_tile_keys`)."""
     Hkv = Hkv if Hkv is not None else Hq // G
     wide = wide and (mask is None or mask.kind == "causal") and wide_tiles_pay(q_lens, G, Hkv, D)
+    tile_keys = WIDE_ROWS if wide else pick_tile_keys(q_lens, G, block_size)
     work, tok_splits, max_splits = plan_attention_work(q_lens, kv_lens, G, causal, Hkv=Hkv,
                                                        seq_rows=seq_rows, allow_split=allow_split,
                                                        mask=mask, align=align,
                                                        rows_per_item=WIDE_ROWS if wide else 128,
-                                                       fill_slots=not wide and pick_tile_keys(q_lens, G) == 64)
+                                                       fill_slots=tile_keys == 64,
+                                                       slots=attention_slots(tile_keys))
     T = int(sum(q_lens))
     n = work.shape[0]
     if work_capacity is not None:
@@ -1033,7 +1041,7 @@ def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, ca
     meta.block_tables = block_tables
     meta.max_splits = max_splits
     meta.num_work = work.shape[0]
-    meta.tile_keys = WIDE_ROWS if wide else pick_tile_keys(q_lens, G)
+    meta.tile_keys = tile_keys
     if max_splits > 1 and dev.type == "cuda":
         meta.o_part = torch.empty(max_splits, T, Hq, D, dtype=torch.float32, device=dev)
         meta.lse_part = torch.empty(max_splits, T, Hq, dtype=torch.float32, device=dev)
@@ -1050,8 +1058,9 @@ class DecodePlan:
         self.G, self.Hq, self.Hkv, self.D, self.bucket = G, Hq, Hkv, D, bucket
         # enough KV splits to occupy the GPU when the batch is small; for a large batch the
         # sequences of the last, partly filled wave of CTAs are cut (tail_split_plan)
-        small_tiles = max_q * G <= 32 and block_size <= 64
-        slots = 148 * (2 if small_tiles else 1)
+        self.tile_keys = pick_tile_keys([max_q], G, block_size)
+        self.slots = slots = attention_slots(self.tile_keys)
+        small_tiles = self.tile_keys == 64
         self.splits = int(max(1, min(16, 148 // max(1, bucket * Hkv))))
         n_cut, pieces = tail_split_plan(bucket, Hkv, slots)
         if self.splits == 1 and n_cut > 0 and max_q == 1:
@@ -1061,7 +1070,6 @@ class DecodePlan:
             self.splits = max(self.splits, 4)
         # pieces that any number of sequences of this bucket can come to
         self.work_cap = 1 + max(self._pieces(n, Hkv, slots, small_tiles) for n in range(1, bucket + 1))
-        self.tile_keys = 64 if small_tiles else 128
         self.meta = AttentionMetadata([], [], bucket)
 
     def _pieces(self, n: int, Hkv: int, slots: int, small: bool) -> int:
@@ -1077,7 +1085,8 @@ class DecodePlan:
     def plan(self, q_lens, kv_lens):
         return plan_attention_work(q_lens, kv_lens, self.G, True, Hkv=self.Hkv,
                                    max_splits_cap=self.splits, mask=self.mask,
-                                   align=self.block_size, fill_slots=self.tile_keys == 64)
+                                   align=self.block_size, fill_slots=self.tile_keys == 64,
+                                   slots=self.slots)
 
     def bind(self, host, dev: torch.Tensor, block_tables: torch.Tensor) -> None:
         """``host`` (numpy) and ``dev``: this plan's ``int32_words`` of the staging buffers."""

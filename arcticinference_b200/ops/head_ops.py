@@ -57,7 +57,8 @@ def build_plan(shape: HeadShape, q_lens, kv_lens, block_tables, block_size, devi
         meta.block_tables = block_tables
         return meta
     return build_attention_metadata(q_lens, kv_lens, block_tables, shape.group, shape.heads, shape.D,
-                                    device, Hkv=shape.kv_heads, mask=shape.mask, align=block_size)
+                                    device, Hkv=shape.kv_heads, mask=shape.mask, align=block_size,
+                                    block_size=block_size)
 
 
 class HeadDecodePlan(DecodePlan):

@@ -1,6 +1,8 @@
 """The host-side planner of attention work items (``ops.plan_attention_work``)."""
 
 import numpy as np
+import pytest
+import torch
 
 from arcticinference_b200 import ops
 
@@ -75,3 +77,39 @@ def test_captured_decode_plan_holds_every_mix_of_requests():
                 work, splits, most = plan.plan(q, kv)
                 assert work.shape[0] <= plan.work_cap and most <= plan.splits
                 _covered(work, len(q), kv) if max(q) == 1 else None
+
+
+@pytest.mark.parametrize("block_size", [16, 64, 128])
+@pytest.mark.parametrize("hkv,G,max_q", [(1, 4, 1), (2, 8, 1), (4, 8, 4), (8, 4, 1), (8, 4, 4), (8, 4, 16), (16, 1, 1),
+                                         (1, 64, 1)])
+def test_captured_decode_plan_holds_every_count_of_requests(block_size, hkv, G, max_q):
+    """Whatever the cache's block size says about the kernel, the work list holds any number of requests, alone,
+    with drafts, and with the padding tokens' sequence."""
+    rng = np.random.default_rng(1)
+    for bucket in (1, 4, 24, 56, 64, 96, 152, 304):
+        plan = ops.DecodePlan(G, G * hkv, hkv, 128, bucket, max_q, block_size)
+        host = np.zeros(plan.int32_words, dtype=np.int32)
+        plan.bind(host, torch.zeros(plan.int32_words, dtype=torch.int32), None)
+        for n in sorted({1, 2, bucket, *range(max(1, bucket - 16), bucket), *rng.integers(1, bucket + 1, 12).tolist()}):
+            for q_lens in ([1] * n, [max_q] * max(1, n // max_q)):
+                for kv in ([2000] * len(q_lens), rng.integers(max_q, 20000, len(q_lens)).tolist()):
+                    q, kv = list(q_lens), list(kv)
+                    if sum(q) > bucket:
+                        continue
+                    if sum(q) < bucket:
+                        q, kv = q + [bucket - sum(q)], kv + [bucket - sum(q)]
+                    work, splits, most = plan.plan(q, kv)
+                    assert work.shape[0] <= plan.work_cap and most <= plan.splits, (bucket, n)
+                    plan.fill(q, kv)
+
+
+def test_plan_and_kernel_agree_on_the_ctas_that_an_sm_holds():
+    """Blocks of 128 tokens take the kernel with one CTA per SM: pieces for 148 CTAs, not for 296."""
+    for n in (1, 8, 18, 40):
+        q, kv = [1] * n, [16384] * n
+        m = {bs: ops.build_attention_metadata(q, kv, None, 4, 32, 128, "cpu", Hkv=8, block_size=bs) for bs in (64, 128)}
+        assert m[64].tile_keys == 64 and m[128].tile_keys == 128
+        for bs, meta in m.items():
+            assert ops.DecodePlan(4, 32, 8, 128, n, 1, bs).tile_keys == meta.tile_keys
+        if n * 8 < 148:
+            assert m[128].num_work * 8 <= 148 and m[64].num_work >= m[128].num_work

@@ -946,7 +946,8 @@ def _plan_decode_work(kv_lens, G, causal, slots, Hkv, seq_rows, allow_split, max
     if allow_split and R * Hkv < slots:
         want = max(1, slots // max(1, R * Hkv))
         if fill_slots:
-            want = decode_splits(R * Hkv, int(key_tiles.mean()), slots, int(min(16, max_splits_cap)))
+            # (never fewer than one wave of CTAs allows: a long sequence among short ones is cut by that alone)
+            want = max(want, decode_splits(R * Hkv, int(key_tiles.mean()), slots, int(min(16, max_splits_cap))))
         cand = np.minimum(np.minimum(16, max_splits_cap), np.minimum(want, np.maximum(1, key_tiles // 2)))
         ns = np.where(key_tiles > 4, cand, 1)
     elif allow_split and max_splits_cap > 1:

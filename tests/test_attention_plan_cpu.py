@@ -113,3 +113,20 @@ def test_plan_and_kernel_agree_on_the_ctas_that_an_sm_holds():
             assert ops.DecodePlan(4, 32, 8, 128, n, 1, bs).tile_keys == meta.tile_keys
         if n * 8 < 148:
             assert m[128].num_work * 8 <= 148 and m[64].num_work >= m[128].num_work
+
+
+def test_long_sequences_among_short_ones_are_cut_as_one_wave_allows():
+    """However short the others are, no piece is longer than with as many pieces per sequence as one wave holds."""
+    rng = np.random.default_rng(2)
+
+    def longest(q_lens, kv, hkv, **kw):
+        work, _, _ = ops.plan_attention_work(q_lens, kv, 4, True, Hkv=hkv, slots=296, **kw)
+        _covered(work, len(kv), kv)
+        return ((work[:, 5] - work[:, 4] + 127) // 128).max()
+
+    cases = [([1] * n, [short] * (n - 1) + [32000], hkv) for n in (16, 24, 36) for hkv in (1, 2, 8) for short in (5, 900)]
+    for _ in range(200):
+        n, q = int(rng.integers(1, 38)), int(rng.choice([1, 4, 8]))
+        cases.append(([q] * n, (2 ** rng.uniform(3, 15, n)).astype(int).tolist(), int(rng.choice([1, 2, 4, 8]))))
+    for q_lens, kv, hkv in cases:
+        assert longest(q_lens, kv, hkv, fill_slots=True) <= longest(q_lens, kv, hkv), (q_lens, kv, hkv)

@@ -45,7 +45,6 @@ def _model_tensors(engine):
 def mark_static_weights(engine) -> None:
     """Tell the linear layers which tensors are parameters (``ops.mark_static``)."""
     from .. import ops
-    ops.clear_static()
     for owner, name in _model_tensors(engine):
         t = _get(owner, name) if (isinstance(owner, dict) and name in owner) or \
             (not isinstance(owner, dict) and hasattr(owner, name)) else None
@@ -78,9 +77,7 @@ def sleep_engine(engine, level: int = 1) -> None:
     engine._sleep_store = {}
     if level == 2:
         seen = {}
-        from .. import ops
         from ..models.quant import Fp8Weight
-        ops.clear_static()
         engine._sleep_shadows = []
         for owner, name in _model_tensors(engine):
             if isinstance(owner, Fp8Weight) and owner.shadow is not None:

@@ -141,21 +141,49 @@ def quant_fp8_row(x: torch.Tensor, sync=None):
     return quant.QuantAct(xq, sx)
 
 
+class StorageSet:
+    """Storages of tensors, by identity: a storage leaves the set when its tensors are gone, and another one at the
+    same address is not in it. (The weak references keep the small objects behind the storages, whose addresses are
+    the keys, from being used again; not their memory.)"""
+
+    def __init__(self):
+        self._refs: dict = {}
+
+    def add(self, t: torch.Tensor) -> None:
+        from torch.multiprocessing.reductions import StorageWeakRef
+        n = len(self._refs)
+        if n & (n - 1) == 0:
+            self._refs = {k: r for k, r in self._refs.items() if not r.expired()}
+        s = t.untyped_storage()
+        self._refs[s._cdata] = StorageWeakRef(s)
+
+    def clear(self) -> None:
+        self._refs.clear()
+
+    def __len__(self) -> int:
+        return len(self._refs)
+
+    def __contains__(self, t: torch.Tensor) -> bool:
+        return bool(self._refs) and t.untyped_storage()._cdata in self._refs
+
+
 # Storages of parameters (weights that no kernel of the compute stream writes). A linear layer
 # whose weight lives in one of them requests its first weight tiles before it waits for the
 # kernel launched before it, so the weight stream starts under that kernel's tail.
-_static_storages: set = set()
+_static_storages = StorageSet()
 
 
 def mark_static(t) -> None:
-    """Declare ``t`` (a tensor or a quantised weight) a parameter. An in-place update of a
-    parameter (a weight sync) is followed by other kernels before the next linear layer that
-    reads it, which is what makes the early read safe."""
+    """Declare ``t`` (a tensor or a quantised weight) a parameter. What is under way on the device is finished
+    first, so it may be the result of any kernel. From then on it is written by copies alone (a weight sync):
+    those signal nothing early, so no kernel behind one reads it too soon, while a kernel of this library lets
+    its successors start before its writes are done."""
     if t is None:
         return
     q = getattr(t, "q", t)
     if isinstance(q, torch.Tensor) and q.is_cuda:
-        _static_storages.add(q.untyped_storage().data_ptr())
+        torch.cuda.synchronize(q.device)
+        _static_storages.add(q)
 
 
 def clear_static() -> None:
@@ -163,7 +191,7 @@ def clear_static() -> None:
 
 
 def _is_static(t: torch.Tensor) -> bool:
-    return bool(_static_storages) and t.untyped_storage().data_ptr() in _static_storages
+    return t in _static_storages
 
 
 def _linear_desc(x, ldx, sx, w, ldw, sw, out_ptr, ldo, M, N, K, bias, residual, act,
@@ -1186,7 +1214,7 @@ def bert_layers(h: torch.Tensor, layers, inter: int, heads: int, D: int, eps: fl
                 meta: AttentionMetadata) -> torch.Tensor:
     """Encoder layers over a packed batch, ``h`` [T, heads * D] (overwritten) in and out, all of them
     enqueued by one native call. ``layers``: a tuple per layer of the weights in the order of
-    ``Ab200BertLayer``, contiguous and of h's type (bf16)."""
+    ``Ab200BertLayer``, contiguous and of h's type (bf16); parameters in the sense of :func:`mark_static`."""
     nat = _native()
     T, H = h.shape
     shapes = ((3 * H, H), (3 * H,), (H, H), (H,), (H,), (H,), (inter, H), (inter,), (H, inter), (H,), (H,), (H,))

@@ -740,6 +740,18 @@ def test_linear_one_row_of_tiles_splits_k_inside_clusters(M, N, K):
     ops.check_status()
 
 
+def test_a_freed_parameter_is_no_parameter():
+    """What is allocated where a parameter lay may be written by a kernel: none of it is read early."""
+    w = _rand(4096, 1024)
+    ops.mark_static(w)
+    assert ops._is_static(w) and ops._is_static(w[:128])
+    at = w.data_ptr()
+    del w
+    w = _rand(4096, 1024)
+    assert w.data_ptr() == at and not ops._is_static(w)
+    ops.clear_static()
+
+
 @pytest.mark.parametrize("splits", [1, 2, 4, 8])
 def test_linear_fp8_row_split_k(splits):
     M, N, K = 24, 1024, 4096

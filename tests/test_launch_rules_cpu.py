@@ -1,12 +1,15 @@
 """Rules of programmatic launches (csrc/common/pdl.cuh) that the sources can be held to by reading: the launch
 trigger of a kernel that allocates tensor memory comes behind the barrier after the allocation, and no
-block leaves a kernel before it has waited for the kernels ahead of it."""
+block leaves a kernel before it has waited for the kernels ahead of it. And which weights may be read ahead of the wait."""
 
 import glob
 import os
 import re
 
 import pytest
+import torch
+
+from arcticinference_b200 import ops
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "arcticinference_b200", "csrc")
 
@@ -54,3 +57,24 @@ def test_no_block_leaves_before_it_has_waited(name, body):
     first_wait = body.index("pdl_wait()")
     for m in re.finditer(r"\breturn;", body):
         assert m.start() > first_wait, name
+
+
+def test_storages_are_known_by_identity():
+    """A parameter that is gone is no parameter any more, whatever is allocated where it lay; views of one are."""
+    known, w = ops.StorageSet(), torch.empty(1 << 20)
+    known.add(w)
+    assert w in known and w[3:7].view(1, -1) in known and torch.empty(8) not in known
+    again = []
+    del w
+    for _ in range(64):
+        again.append(torch.empty(1 << 20))
+        assert again[-1] not in known
+    for i in range(64):        # (addresses of the objects behind the storages are not used again either)
+        t = torch.empty(16 + i)
+        known.add(t)
+        del t
+        assert torch.empty(16 + i) not in known
+    known.add(again[0])
+    assert again[0] in known and len(known) <= 64 + 2
+    known.clear()
+    assert again[0] not in known

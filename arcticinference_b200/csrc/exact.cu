@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(256) linear_exact_kernel(const ExactArgs p) {
     group = t.x;
     row0 = t.y;
     nrows = t.z;
+    if (nrows <= 0) return;   // (lists for pairs of tiles are filled up with empty ones)
   } else {
     group = blockIdx.z;
     row0 = blockIdx.y * kXM;

@@ -34,6 +34,7 @@ struct GroupedArgs {
   int M, m_tiles, groups;   // without a tile list: rows and row tiles per group
   int x_by_group;           // the activations' map has a group dimension
   int m_fastest;            // work order: row tiles of one weight tile next to each other
+  int skip_empty;           // the list was filled up for pairs of tiles, which these products do not take
   int act;
   GateParams gate;
   uint32_t tmem_cols;
@@ -179,6 +180,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
       bool ok = true;
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
         const GgWork t = gg_work(p, w, m_total);
+        if (p.skip_empty && t.nrows <= 0) continue;
         const bool few = t.nrows <= 32;
         const uint32_t bytes = b_bytes + (few ? 32u * kGgBlockK * 2u : kGgABytes);
         const int xg = p.x_by_group ? t.group : 0;
@@ -222,6 +224,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
     uint32_t phase = 0, acc_phase = 0;
     bool ok = true;
     for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+      if (p.skip_empty && gg_work(p, w, m_total).nrows <= 0) continue;
       if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status,
                                              1200 + acc, w)))
         break;
@@ -262,6 +265,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
     uint32_t acc_phase = 0;
     for (int w = blockIdx.x; w < total_work; w += gridDim.x) {
       const GgWork t = gg_work(p, w, m_total);
+      if (p.skip_empty && t.nrows <= 0) continue;
       const int n0 = t.nt * p.bn;
       if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status,
                                              1400 + acc, w)))
@@ -527,6 +531,7 @@ int ab200_grouped_gemm(const void* x, long long ldx, long long x_gstride, long l
   if (a.stages > kGgMaxStages) a.stages = kGgMaxStages;
 
   const bool pair = pairs != 0 && tiles != nullptr && a.bn == 256;
+  a.skip_empty = pairs != 0 && !pair;
   CUtensorMap tx, tx32, tw;
   {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)x_rows, (uint64_t)(a.x_by_group ? groups : 1)};

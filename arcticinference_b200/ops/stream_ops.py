@@ -362,7 +362,11 @@ def route_ref(x, w, b, top: int, scale=None, groups=None):
     return order, torch.softmax(z.gather(1, order), -1)
 
 
-PAIR_MIN_ROWS = 640    # rows per expert on average: half a tile of padding is 8 % there, 5 to 10 % less time
+# Rows per expert on average from which the lists are made for pairs of tiles. Half a tile of padding per expert is
+# 8 % there. Both products of a 2048-wide layer, single tiles and pairs, us: 64 experts of 2 x 1408, 512 rows each
+# 549 and 487, 640: 710 and 634, 768: 829 and 723, 1024: 1083 and 932, 2048: 2149 and 1574; 8 experts of 2 x 2816,
+# 512 rows 183 and 186, 640: 236 and 208, 1024: 256 and 220. Below, what is left of the last tiles decides.
+PAIR_MIN_ROWS = 640
 
 _route_states: dict = {}
 

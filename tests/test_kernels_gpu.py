@@ -469,8 +469,8 @@ def test_attention_merge_pieces(T, ns):
 
 
 # experts on pairs of tiles: odd and even numbers of tiles, an expert without rows, K and N that end inside a
-# block and a tile
-@pytest.mark.parametrize("N,K", [(512, 256), (800, 136)])
+# block and a tile; and the kernel with single tiles, which takes narrow products of the same lists
+@pytest.mark.parametrize("N,K", [(512, 256), (800, 136), (64, 256), (128, 136)])
 @pytest.mark.parametrize("act", [None, "silu"])
 def test_grouped_linear_pairs(N, K, act):
     from arcticinference_b200.ops import stream_ops as st
@@ -482,11 +482,15 @@ def test_grouped_linear_pairs(N, K, act):
     w = _rand(E, N, K, scale=1.0 / math.sqrt(K))
     out = st.grouped_linear(rows, w, r, act=act)
     ops.check_status()
+    # weights whose rows are no multiple of 16 bytes apart take the kernel without tensor cores: the same list
+    loose = torch.empty(E, N, K + 1, dtype=w.dtype, device=DEV)[:, :, :K].copy_(w)
+    exact = st.grouped_linear(rows, loose, r)
     expert = torch.empty(T * top, dtype=torch.long, device=DEV)
     expert[r.rows.long().reshape(-1)] = r.ids.long().reshape(-1)
     z = torch.zeros(T * top, N, dtype=torch.float64, device=DEV)
     for e in range(E):
         z[expert == e] = rows[expert == e].double() @ w[e].double().t()
+    assert ((exact.double() - z).abs() <= z.abs() * 2.0 ** -8 + 2e-4).all()
     if act:
         g, u = (t.flatten(1) for t in z.view(T * top, N // 32, 2, 16).unbind(2))
         z = torch.nn.functional.silu(g) * u

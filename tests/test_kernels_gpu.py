@@ -258,6 +258,24 @@ def test_linear_few_tokens(M, N, K, fp8):
     _check_linear(M, N, K, fp8)
 
 
+@pytest.mark.parametrize("M", [1, 200, 257])
+def test_linear_gelu_values(M):
+    """GELU of every bf16 magnitude, infinities and NaN (as biases of empty products): few tokens, two
+    accumulators, CTA pairs."""
+    bits = torch.arange(0x8000, dtype=torch.int32, device=DEV)
+    b = torch.cat([bits, bits + 0x8000]).to(torch.int16).view(torch.bfloat16)
+    out = ops.linear(torch.zeros(M, 16, dtype=b.dtype, device=DEV), torch.zeros(b.numel(), 16, dtype=b.dtype, device=DEV),
+                     bias=b, act="gelu")
+    ops.check_status()
+    v = b.double()
+    y = v * (0.5 * torch.special.erfc(-v / math.sqrt(2)))     # (-inf times 0 is no number)
+    assert torch.equal(out.isnan(), y.isnan().expand(M, -1)) and y.isnan().sum() > 2 * 127
+    # one rounding to bf16; 8e-6 of the value from the tail's exponential; results below the normal numbers are lost
+    bound = y.abs() * (2.0 ** -8 + 8e-6) + 2.0 ** -126
+    ok = ((out.double() - y).abs() <= bound) | y.isnan() | (out.double() == y)
+    assert ok.all(), b[~ok.all(0)][:8]
+
+
 # gate / up rows of one tile in the two CTAs of a pair: ends of the tiles, more tiles than pairs
 @pytest.mark.parametrize("M,inter,K", [(257, 128, 64), (300, 136, 80), (513, 1416, 768), (5000, 2040, 256)])
 def test_linear_silu(M, inter, K):

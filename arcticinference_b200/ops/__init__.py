@@ -1217,6 +1217,8 @@ def bert_layers(h: torch.Tensor, layers, inter: int, heads: int, D: int, eps: fl
     ``Ab200BertLayer``, contiguous and of h's type (bf16); parameters in the sense of :func:`mark_static`."""
     nat = _native()
     T, H = h.shape
+    if T == 0:
+        return h
     shapes = ((3 * H, H), (3 * H,), (H, H), (H,), (H,), (H,), (inter, H), (inter,), (H, inter), (H,), (H,), (H,))
     for lw in layers:
         for t, shape in zip(lw, shapes, strict=True):
@@ -1227,7 +1229,7 @@ def bert_layers(h: torch.Tensor, layers, inter: int, heads: int, D: int, eps: fl
     rc = nat.lib().ab200_bert_layers(
         ptrs, len(layers), h.data_ptr(), x.data_ptr(), wide.data_ptr(), a.data_ptr(), T, H, inter, heads,
         D, float(eps), meta.work.data_ptr(), meta.num_work,
-        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128, max(max(meta.q_lens), max(meta.kv_lens)),
+        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128, max(meta.q_lens + meta.kv_lens),
         nat.status_buffer(h.device).data_ptr(), nat.stream_ptr())
     nat.check(rc, "bert_layers T=%d" % T)
     launch_counter.add(7 * len(layers))
@@ -1250,7 +1252,7 @@ def attention_contiguous(q, k, v, seq_lens, H: int, D: int, scale: float | None 
     if out is None:
         out = torch.empty(T, H * D, dtype=q.dtype, device=q.device)
     assert k.stride(0) == v.stride(0)
-    longest = max(max(meta.q_lens), max(meta.kv_lens))
+    longest = max(meta.q_lens + meta.kv_lens, default=0)
     if not causal and D == 64 and longest <= SHORT_TOKENS:
         rc = nat.lib().ab200_attention_short(
             q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), meta.work.data_ptr(),

@@ -469,6 +469,19 @@ def test_bert_layers_native(seq_lens):
     ops.check_status()
 
 
+def test_encoder_calls_without_tokens():
+    from arcticinference_b200.config import ModelConfig
+    from arcticinference_b200.models.bert import BertEncoder
+    for seq_lens in ([], [0, 0]):
+        out = ops.attention_contiguous(*(_rand(0, 192) for _ in range(3)), seq_lens, 3, 64)
+        assert out.shape == (0, 192)
+    enc = BertEncoder(ModelConfig.from_pretrained("bert-tiny"), DEV, torch.bfloat16)
+    enc.init_random()
+    none = torch.empty(0, dtype=torch.int64, device=DEV)
+    assert enc.forward(none, none, []).shape == (0, enc.cfg.hidden_size)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("T,ns", [(1, 16), (3, 1), (5, 5), (700, 3)])
 def test_attention_merge_pieces(T, ns):
     Hq, Hkv, D, n = 6, 2, 128, 140

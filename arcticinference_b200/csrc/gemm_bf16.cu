@@ -1295,8 +1295,7 @@ static FewPlan few_plan_of(int tokens, int N, int kblocks, int group_max, int sm
   std::lock_guard<std::mutex> lock(mu);
   auto it = plans.find(key);
   if (it != plans.end()) return it->second;
-  const FewPlan plan = plan_few(M, N, kblocks, group_max, sms,
-                                cluster_splits_off() ? [](int, size_t) { return 0; } : cluster_capacity);
+  const FewPlan plan = plan_few(M, N, kblocks, group_max, sms, cluster_capacity);
   if (plans.size() > 8192) plans.clear();
   plans.emplace(key, plan);
   return plan;
@@ -1405,7 +1404,8 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
   }
 
   const bool alone = sync == nullptr || (sync->wait_world == 0 && sync->sig_world == 0);
-  if (M <= 256 && peer_cols == 0 && alone && force_splits == 0 &&
+  // (that kernel splits K in clusters alone; without them the general one does, through the workspace)
+  if (M <= 256 && peer_cols == 0 && alone && force_splits == 0 && !cluster_splits_off() &&
       (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
     const int elems = fp8 ? kBlockKFp8 : kBlockK;
     const int kblocks = (K + elems - 1) / elems;

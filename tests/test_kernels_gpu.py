@@ -1,6 +1,9 @@
 """Numerics of the sm_100a kernels against plain PyTorch fp32 restatements."""
 
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -256,6 +259,28 @@ def _check_linear(M, N, K, fp8):
                                    (255, 4096, 14336), (256, 32000, 512)])
 def test_linear_few_tokens(M, N, K, fp8):
     _check_linear(M, N, K, fp8)
+
+
+def test_linear_few_tokens_without_clusters():
+    """AB200_GEMM_CLUSTER=0 splits K through the workspace. The switch is read once: a process of its own."""
+    code = """
+import torch
+from arcticinference_b200 import ops
+from arcticinference_b200.ops import native
+torch.manual_seed(0)
+x, w = (torch.randn(n, 3072, device="cuda:0").bfloat16() for n in (50, 768))
+ws = native.workspace(x.device)
+ws.zero_()
+y = ops.linear(x, w / 64)
+ops.check_status()
+assert ws.any(), "K was not split"
+z = x.double() @ (w / 64).double().t()
+assert ((y.double() - z).abs() <= z.abs() * 2.0 ** -8 + 2e-4).all()
+"""
+    env = dict(os.environ, AB200_GEMM_CLUSTER="0", ARCTIC_B200_NO_AUTOBUILD="1",
+               PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    run = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
 
 
 @pytest.mark.parametrize("M", [1, 200, 257])

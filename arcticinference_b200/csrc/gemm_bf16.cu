@@ -1258,26 +1258,24 @@ static double plan_cost_us(int tiles, int splits, int kblocks, int capacity, boo
   return t;
 }
 
-// Cycles that an SM spends on one k-block of a 128 x bn tile: the tensor core's (2 per column), or
+// Cycles that a CTA of a pair spends on one k-block of a 256 x bn tile: the tensor core's (2 per column), or
 // what its shared memory takes to receive and to read the operands (128 bytes a cycle).
-static double kblock_cycles(int bn, int staged_b_rows) {
-  const double mma = 2.0 * bn, smem = 2.0 * (kABytes + 128.0 * staged_b_rows) / 128.0;
+static double pair_kblock_cycles(int bn) {
+  const double mma = 2.0 * bn, smem = 2.0 * (kABytes + 64.0 * bn) / 128.0;
   return mma > smem ? mma : smem;
 }
 
-// Width of the tiles that a product of more than one row of tiles is cut into, for `units` CTAs or
-// pairs that work at a time: the one with the least time in whole waves.
-static int pick_tile_width(int tiles_a, int N, int kblocks, int units, bool pair, double* cycles) {
+// Width of the tiles that a product on `pairs` pairs of CTAs is cut into: the one with the least time in whole waves.
+static int pick_pair_width(int tiles_a, int N, int kblocks, int pairs) {
   int best = 0;
+  double cycles = 0;
   for (int bn = 256; bn >= 128; bn -= 64) {
     if (bn > 128 && bn > ((N + 63) / 64) * 64) continue;
-    if (!pair && bn == 192) continue;
     const long long tiles = (long long)tiles_a * ((N + bn - 1) / bn);
-    const double t = (double)((tiles + units - 1) / units) *
-                     (kblocks * kblock_cycles(bn, pair ? bn / 2 : bn) + 1000.0);
-    if (best == 0 || t < *cycles) {
+    const double t = (double)((tiles + pairs - 1) / pairs) * (kblocks * pair_kblock_cycles(bn) + 1000.0);
+    if (best == 0 || t < cycles) {
       best = bn;
-      *cycles = t;
+      cycles = t;
     }
   }
   return best;
@@ -1604,14 +1602,14 @@ static int launch_linear(const void* x, long long ldx, const void* w, long long 
                (reinterpret_cast<uintptr_t>(bias) % 16) == 0 &&
                (residual == nullptr || ldr % 8 == 0);
 
-  // More than one row of tiles: CTA pairs, unless the tiles of single CTAs fill the GPU better.
+  // More than one row of tiles: CTA pairs. Also where tiles of single CTAs would come in one wave and those of pairs
+  // in two: 6272 x 768 x 3072 28.7 us on pairs, 33.3 on single CTAs with tiles of 256 columns, 53 of 128; 1100 x 4096
+  // x 4096 35.6, 40.2 and 67; 1152 x 4096 x 14336 119, 121 and 210.
   if (!a.transposed && a.tiles_a > 1 && M > 256 && N >= 128 && peer_cols == 0 && alone && !w_tiled &&
       a.coalesce) {
-    double single = 0, paired = 0;
-    pick_tile_width(a.tiles_a, N, a.kblocks_total, sms, false, &single);
     const int tiles_pair = (M + 2 * kBlockM - 1) / (2 * kBlockM);
-    const int bn = pick_tile_width(tiles_pair, N, a.kblocks_total, sms / 2, true, &paired);
-    if ((gate_rows > 0 || paired <= single) && cluster_capacity(2, 227 * 1024 - 1024) > 0) {
+    const int bn = pick_pair_width(tiles_pair, N, a.kblocks_total, sms / 2);
+    if (cluster_capacity(2, 227 * 1024 - 1024) > 0) {
       a.gate_rows = gate_rows;
       a.bn = bn;
       a.tiles_a = tiles_pair;

@@ -1028,17 +1028,41 @@ SHORT_TOKENS = 128   # longest sequence of the kernel for many short ones
 WIDE_ROWS = 256   # rows of a work item of the kernel with two tiles of rows per CTA
 
 
-def wide_tiles_pay(q_lens, G: int, Hkv: int, D: int, num_sms: int = 148) -> bool:
-    """Whether a call should take 256 query rows per CTA. A CTA with two tiles takes 1.35 times as long as
-    one with a single tile and there are half as many of them, unless sequences are short: it pays
-    wherever the waves of CTAs become fewer (measured: 61 decodes beside 1987 tokens, 7 waves and 6, 159
-    and 140 us; four texts of 2048, 14 and 7, 291 and 186), and not in a single wave."""
-    tpt = 128 // G
-    if D not in (64, 128) or max(q_lens, default=0) <= tpt:
+# us of a CTA of 128 query rows and of one of 256: (its set-up, per 128-key tile, per tile where the second 128 rows
+# are empty, part of a mean CTA that the end of the call adds)
+_ATTENTION_US = {64: ((5.0, 1.4, 1.4, 0.6), (5.3, 1.9, 1.45, 0.5)),
+                 128: ((6.5, 1.6, 1.6, 0.25), (7.5, 2.0, 1.5, 0.25))}
+
+
+def _attention_us(q, kv, G: int, Hkv: int, causal: bool, rows: int, costs, num_sms: int) -> float:
+    """Time of a call whose CTAs take ``rows`` query rows: its longest CTA's or, if that is more, the mean load of
+    an SM and the end of the call."""
+    setup, pair, lone, tail = costs
+    tokens = rows // G
+    n = -(-q // tokens)
+    seq = np.repeat(np.arange(q.size), n)
+    first = (np.arange(seq.size) - (np.cumsum(n) - n)[seq]) * tokens     # of a CTA's tokens in its sequence
+    last = np.minimum(first + tokens, q[seq])
+    keys = (kv - q)[seq] + last if causal else kv[seq]
+    us = setup + -(-keys // TILE_KEYS) * np.where(last - first > 128 // G, pair, lone)
+    return max(float(us.max()), float(us.sum()) * Hkv / num_sms + tail * float(us.mean()))
+
+
+def wide_tiles_pay(q_lens, kv_lens, G: int, Hkv: int, D: int, causal: bool = True, num_sms: int = 148) -> bool:
+    """Whether a call should take 256 query rows per CTA: half as many CTAs for the rows of prompts, each up to 1.4
+    times as long. Not where single tiles leave SMs without one, and otherwise where the estimate is the lower. The
+    costs are fitted (5 % off) to 86 random steps of prompts and decodes, 1 to 16 key heads, up to 11 CTAs per SM, each
+    run both ways: single tiles 6709 us in all, two tiles 5172, this rule 5078, the better way each time 5055, no step
+    more than 1.11 times its single tiles. Long prompts gain (3888 tokens, 8 key heads 229 -> 129 us), a lone longest
+    CTA loses (3695 tokens, 2 key heads 53 -> 65 us) and keeps single tiles."""
+    if D not in _ATTENTION_US or max(q_lens, default=0) <= 128 // G:
         return False
-    one = sum(-(-q // tpt) for q in q_lens) * Hkv
-    two = sum(-(-q // (2 * tpt)) for q in q_lens) * Hkv
-    return -(-two // num_sms) < -(-one // num_sms)
+    q, kv = np.asarray(q_lens, dtype=np.int64), np.asarray(kv_lens, dtype=np.int64)
+    if int((-(-q // (128 // G))).sum()) * Hkv <= num_sms:
+        return False
+    single, wide = (_attention_us(q, kv, G, Hkv, causal, rows, costs, num_sms)
+                    for rows, costs in zip((128, WIDE_ROWS), _ATTENTION_US[D]))
+    return wide < 0.97 * single
 
 
 def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, causal=True,
@@ -1049,7 +1073,7 @@ def build_attention_metadata(q_lens, kv_lens, block_tables, G, Hq, D, device, ca
     (:func:`attention`, :func:`attention_contiguous`), so the better one may be chosen. ``block_size``: the
     paged cache's, which decides on the kernel (:func:`pick_tile_keys`)."""
     Hkv = Hkv if Hkv is not None else Hq // G
-    wide = wide and (mask is None or mask.kind == "causal") and wide_tiles_pay(q_lens, G, Hkv, D)
+    wide = wide and (mask is None or mask.kind == "causal") and wide_tiles_pay(q_lens, kv_lens, G, Hkv, D, causal)
     tile_keys = WIDE_ROWS if wide else pick_tile_keys(q_lens, G, block_size)
     work, tok_splits, max_splits = plan_attention_work(q_lens, kv_lens, G, causal, Hkv=Hkv,
                                                        seq_rows=seq_rows, allow_split=allow_split,

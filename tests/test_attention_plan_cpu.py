@@ -130,3 +130,16 @@ def test_long_sequences_among_short_ones_are_cut_as_one_wave_allows():
         cases.append(([q] * n, (2 ** rng.uniform(3, 15, n)).astype(int).tolist(), int(rng.choice([1, 2, 4, 8]))))
     for q_lens, kv, hkv in cases:
         assert longest(q_lens, kv, hkv, fill_slots=True) <= longest(q_lens, kv, hkv), (q_lens, kv, hkv)
+
+
+# steps that were timed both ways, and by how much two tiles per CTA were the slower or the faster form
+@pytest.mark.parametrize("q_lens,kv_lens,G,hkv,D,wide", [
+    ([1474, 13], [1474, 84], 1, 16, 128, False),                                               # 1.17 times
+    ([1] * 29 + [4, 384, 84, 160, 25, 116], [900] * 29 + [7, 6192, 86, 5315, 25, 159], 8, 2, 64, False),   # 1.21
+    ([634, 3247], [634, 3247], 4, 2, 128, False), ([71, 4029], [71, 4029], 8, 1, 128, False),  # 1.23, 1.25
+    ([2048] * 4, [2048] * 4, 4, 8, 128, True), ([3888], [3888], 4, 8, 128, True),              # 0.64, 0.57
+    ([8192], [32768], 4, 8, 128, True), ([1] * 61 + [1987], [1500] * 61 + [1987], 4, 8, 128, True),        # 0.67, 0.88
+    ([1] * 200, [2000] * 200, 4, 8, 128, False), ([], [], 4, 8, 128, False),
+])
+def test_two_tiles_of_rows_where_they_are_faster(q_lens, kv_lens, G, hkv, D, wide):
+    assert ops.wide_tiles_pay(q_lens, kv_lens, G, hkv, D) == wide

@@ -365,7 +365,8 @@ int ab200_attention_short(const void* q, long long ldq, const void* k, const voi
 
 // All layers of an encoder over a packed batch: h [T, hidden] in and out; x [T, hidden], a [T, hidden]
 // and wide [T, max(3 hidden, inter)] are scratch. One call enqueues the seven kernels of every layer:
-// from Python each launch costs 17 us of the host, more than the kernel takes for a short text.
+// from Python each launch costs 17 us of the host, more than the kernel takes for a short text. max_len > 0: heads of 64
+// take the kernel for short sequences, of which this is the longest.
 int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void* x, void* wide, void* a,
                       int T, int hidden, int inter, int heads, int D, float eps, const void* work,
                       int num_work, int tile_keys, int max_len, int* status, cudaStream_t stream) {
@@ -399,7 +400,7 @@ int ab200_bert_layers(const Ab200BertLayer* layers, int n_layers, void* h, void*
     const Ab200BertLayer& w = layers[l];
     int rc = linear(h, w.wqkv, w.bqkv, wide, 3 * hidden, hidden, 0, nullptr);
     if (rc != 0) return rc;
-    rc = D == kShortDim && max_len <= kShortLen
+    rc = D == kShortDim && max_len > 0
              ? ab200_attention_short(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, work, num_work,
                                      heads, max_len, scale, a, hidden, stream)
              : ab200_attention(qkv, 3 * hidden, qkv + part, qkv + 2 * part, 3 * hidden, T, 0, nullptr, 0, work,

@@ -1025,6 +1025,15 @@ def attention_slots(tile_keys: int, num_sms: int = 148) -> int:
 
 
 SHORT_TOKENS = 128   # longest sequence of the kernel for many short ones
+
+
+def short_attention_pays(longest: int, ctas: int, num_sms: int = 148) -> bool:
+    """Whether an encoder call takes the kernel for short sequences: up to 64 tokens always (2.9 to 4.6 us while
+    the other one takes 6 to 7), up to 128 where the other kernel's CTAs, one per SM, come in more than one wave
+    (16 texts of 128, 12 heads: 9.7 us and 11.4; within one wave 8.0 and 6.0)."""
+    return longest <= SHORT_TOKENS and (longest <= 64 or ctas > num_sms)
+
+
 WIDE_ROWS = 256   # rows of a work item of the kernel with two tiles of rows per CTA
 
 
@@ -1250,10 +1259,12 @@ def bert_layers(h: torch.Tensor, layers, inter: int, heads: int, D: int, eps: fl
     ptrs = (ctypes.c_void_p * (len(layers) * len(shapes)))(*[t.data_ptr() for lw in layers for t in lw])
     x, a = torch.empty_like(h), torch.empty_like(h)
     wide = torch.empty(T, max(3 * H, inter), dtype=h.dtype, device=h.device)
+    longest = max(meta.q_lens + meta.kv_lens)
     rc = nat.lib().ab200_bert_layers(
         ptrs, len(layers), h.data_ptr(), x.data_ptr(), wide.data_ptr(), a.data_ptr(), T, H, inter, heads,
         D, float(eps), meta.work.data_ptr(), meta.num_work,
-        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128, max(meta.q_lens + meta.kv_lens),
+        meta.tile_keys if meta.tile_keys == WIDE_ROWS else 128,
+        longest if short_attention_pays(longest, meta.num_work * heads) else 0,
         nat.status_buffer(h.device).data_ptr(), nat.stream_ptr())
     nat.check(rc, "bert_layers T=%d" % T)
     launch_counter.add(7 * len(layers))
@@ -1277,7 +1288,7 @@ def attention_contiguous(q, k, v, seq_lens, H: int, D: int, scale: float | None 
         out = torch.empty(T, H * D, dtype=q.dtype, device=q.device)
     assert k.stride(0) == v.stride(0)
     longest = max(meta.q_lens + meta.kv_lens, default=0)
-    if not causal and D == 64 and longest <= SHORT_TOKENS:
+    if not causal and D == 64 and short_attention_pays(longest, meta.num_work * H):
         rc = nat.lib().ab200_attention_short(
             q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), meta.work.data_ptr(),
             meta.num_work, H, longest, float(scale), out.data_ptr(), out.stride(0), nat.stream_ptr())

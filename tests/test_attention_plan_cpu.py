@@ -143,3 +143,8 @@ def test_long_sequences_among_short_ones_are_cut_as_one_wave_allows():
 ])
 def test_two_tiles_of_rows_where_they_are_faster(q_lens, kv_lens, G, hkv, D, wide):
     assert ops.wide_tiles_pay(q_lens, kv_lens, G, hkv, D) == wide
+
+
+def test_kernel_of_short_texts_within_a_wave():
+    for longest, ctas, pays in ((1, 12, True), (64, 12, True), (65, 148, False), (128, 149, True), (129, 4000, False)):
+        assert ops.short_attention_pays(longest, ctas) == pays

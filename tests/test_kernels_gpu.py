@@ -457,7 +457,8 @@ def test_paged_attention_wide(q_lens, kv_lens, Hq, Hkv, D, bs, split, monkeypatc
 
 # sequences of at most 128 tokens: every register size, ends of 16-row and 16-key groups
 @pytest.mark.parametrize("seq_lens", [[1], [32, 1, 31], [33, 17, 64, 50], [65, 96, 2], [97, 128, 127, 112]])
-def test_encoder_attention_short(seq_lens):
+def test_encoder_attention_short(seq_lens, monkeypatch):
+    monkeypatch.setattr(ops, "short_attention_pays", lambda longest, ctas: True)
     H, D, T = 3, 64, sum(seq_lens)
     qkv = _rand(T, 3 * H * D)
     out = ops.attention_contiguous(qkv[:, :H * D], qkv[:, H * D:2 * H * D], qkv[:, 2 * H * D:], seq_lens, H, D)

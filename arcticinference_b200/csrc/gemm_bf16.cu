@@ -1,19 +1,19 @@
 // bf16 linear layer  out[M,N] = x[M,K] * w[N,K]^T  (+bias)(+residual)(activation)
-// for sm_100a: a persistent, warp-specialised kernel in which one thread issues
-// tcgen05.mma (UMMA 128 x bn x 16, fp32 accumulators in tensor memory), one
-// thread feeds a ring of 128B-swizzled shared-memory stages with TMA, and four
-// epilogue warps drain the double-buffered TMEM accumulators with tcgen05.ld.
+// for sm_100a, in three warp-specialised kernels: one warp feeds a ring of 128B-swizzled shared-memory
+// stages with TMA, one walks the k-blocks with warp-uniform values while an elected lane issues tcgen05.mma
+// (fp32 accumulators in tensor memory), and eight epilogue warps drain the accumulators with tcgen05.ld.
+//   * gemm_few_kernel (common/gemm_few.cuh), M <= 256: the weights are streamed once, K is split over the
+//     CTAs of a cluster;
+//   * gemm_pair_kernel, M > 256: two CTAs on one tile of 256 rows (cta_group::2), persistent, accumulators
+//     double-buffered, compiled once per kind of epilogue;
+//   * gemm_bf16_kernel, what those two leave: outputs scattered to ranks, ordering between ranks, forced
+//     splits, tiled fp8 weights of many rows, narrow or oddly aligned operands. Persistent single CTAs in two
+//     orientations: token-major (A = 128 tokens, B = bn features), and for 129 .. 256 tokens feature-major
+//     (A = 128 features, B = all tokens; the accumulator holds out^T and the epilogue stores it transposed).
+//     Split-K partial sums go through a cluster's shared memory or to an fp32 scratch buffer supplied by the
+//     caller, which a second kernel folds.
 //
-// Two orientations share the kernel:
-//   * token-major  (M > 256): A operand = x tile (128 tokens), B = w tile (bn features)
-//   * feature-major (M <= 256, decode): A operand = w tile (128 features), B = all
-//     tokens (bn = M rounded up to 16); the accumulator holds out^T and the
-//     epilogue stores it transposed. Every SM then streams weights even when
-//     only a handful of tokens are in flight, and split-K adds parallelism when
-//     N/128 alone cannot fill 148 SMs. Split-K partial sums go to an fp32
-//     scratch buffer supplied by the caller and are folded by a second kernel.
-//
-// The same kernel runs W8A8 fp8 linears whose scales are one per token and one per output
+// The same kernels run W8A8 fp8 linears whose scales are one per token and one per output
 // feature (ab200_linear_fp8_row): the operands are e4m3 bytes (a 128-byte swizzle atom is then
 // 128 k-elements and one kind::f8f6f4 instruction covers 32 of them), the whole K loop
 // accumulates in tensor memory with no rescaling on the way, and the epilogue multiplies each

@@ -873,8 +873,9 @@ class AttentionMetadata:
 def decode_splits(ctas: int, key_tiles: int, slots: int, most: int = 16) -> int:
     """Pieces that each of ``ctas`` equal CTAs of a decode call (two per SM, 64-key stages) should be cut
     into. A CTA streams a 128-key tile in 3 us however few run beside it (all slots together then
-    stream at the copy bandwidth) and costs 4 us besides; pieces cost a merge. 192 CTAs of 24 tiles on 296
-    slots: 67 us whole, 62 in three. At most two waves of pieces."""
+    stream at the copy bandwidth) and costs 4 us besides; pieces cost a merge. On 296 slots, 192 CTAs of 24
+    tiles: 67 us whole, 62 in three; 160 of 4 to 32 tiles 77 whole and 45 in three, 192 of them 81 and 51. At most two
+    waves of pieces."""
     best, best_us = 1, 0.0
     for ns in range(1, max(1, min(most, key_tiles // 2, 2 * slots // max(1, ctas))) + 1):
         us = -(-ctas * ns // slots) * (-(-key_tiles // ns) * 3.0 + 4.0) + (3.0 if ns > 1 else 0.0)

@@ -305,7 +305,7 @@ def test_fp8_engine_matches_the_cpu_path(scheme):
 def test_programmatic_dependent_launch_gives_the_same_tokens():
     """AB200_PDL=1 launches the serving kernels with programmatic stream serialisation (set-up
     and the first weight tiles of a kernel overlap the tail of the one before it). The switch is
-    read once per process, so the opted-in run is a child process; greedy tokens must agree."""
+    read once per process, so both runs are child processes; greedy tokens must agree."""
     import json
     import os
     import subprocess

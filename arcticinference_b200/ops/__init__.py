@@ -174,15 +174,15 @@ _static_storages = StorageSet()
 
 
 def mark_static(t) -> None:
-    """Declare ``t`` (a tensor or a quantised weight) a parameter. What is under way on the device is finished
-    first, so it may be the result of any kernel. From then on it is written by copies alone (a weight sync):
-    those signal nothing early, so no kernel behind one reads it too soon, while a kernel of this library lets
-    its successors start before its writes are done."""
+    """Declare ``t`` (a tensor or a quantised weight) a parameter. It may be the result of any kernel of the
+    current stream: a kernel that signals nothing early is put behind them, which no later one passes. From then
+    on it is written by copies alone (a weight sync), which signal nothing early either, while a kernel of this
+    library lets its successors start before its writes are done."""
     if t is None:
         return
     q = getattr(t, "q", t)
     if isinstance(q, torch.Tensor) and q.is_cuda:
-        torch.cuda.synchronize(q.device)
+        torch.empty(1, device=q.device).zero_()
         _static_storages.add(q)
 
 
